@@ -691,6 +691,7 @@ uint64_t footprint(const lbm_config& c, int64_t* cap_out) {
   b += np * 15 * 3 * 8;
   b += np * (uint64_t)cap * (4 + 8 + 8) + np * 4;
   b += np * (kSweepBytes + 3 * 4);                       // nearest-image sweeps
+  b += np * ((es == 8 ? 6ull * kBounceSplit * 8 : 0) + 4);  // bounce-back partial sums
   if (np > 0) b += 2ull * std::max<uint64_t>(4096, 256 * np) * 4 + 4;  // refill list
   if (c.forcing == LBM_FORCING_STOCHASTIC) {
     b += 3ull * kRowCoef * c.ny * c.nz * es + 45ull * c.nz * 2 * 8;  // row tables, z table
@@ -1014,6 +1015,9 @@ int lbm_create(const lbm_config* cfg, lbm_ctx** out) {
     al((void**)&ctx->links.count, (size_t)ctx->npmax * sizeof(int32_t));
     al(&ctx->links.sweeps, (size_t)ctx->npmax * kSweepBytes);
     al((void**)&ctx->links.sweep_ok, (size_t)ctx->npmax * 3 * sizeof(int32_t));
+    if (!ctx->f32)
+      al((void**)&ctx->links.bsum, (size_t)ctx->npmax * 6 * kBounceSplit * sizeof(double));
+    al((void**)&ctx->links.bdone, (size_t)ctx->npmax * sizeof(int32_t));
     ctx->fill.cap = std::max(4096, 256 * ctx->npmax);
     al((void**)&ctx->fill.node, (size_t)ctx->fill.cap * sizeof(int32_t));
     al((void**)&ctx->fill.part, (size_t)ctx->fill.cap * sizeof(int32_t));
@@ -1032,6 +1036,7 @@ int lbm_create(const lbm_config* cfg, lbm_ctx** out) {
     for (int i = 0; i < 15; ++i) *vecs[i] = b + i * v;
     cudaMemsetAsync(ctx->pbuf, 0, 15 * v * sizeof(double), ctx->stream);
     cudaMemsetAsync(ctx->links.count, 0, ctx->npmax * sizeof(int32_t), ctx->stream);
+    cudaMemsetAsync(ctx->links.bdone, 0, ctx->npmax * sizeof(int32_t), ctx->stream);
     cudaMemsetAsync(ctx->first_move, 0, sizeof(int), ctx->stream);
   }
   cudaMemsetAsync(ctx->f[0], 0, 19 * N * ctx->esz, ctx->stream);
@@ -1142,7 +1147,7 @@ int lbm_destroy(lbm_ctx* ctx) {
                   ctx->rowtab[0], ctx->rowtab[1],
                   ctx->rowtab[2], ctx->pbuf, ctx->first_move, ctx->links.code,
                   ctx->links.alpha, ctx->links.f9, ctx->links.count, ctx->links.sweeps,
-                  ctx->links.sweep_ok, ctx->fill.node,
+                  ctx->links.sweep_ok, ctx->links.bsum, ctx->links.bdone, ctx->fill.node,
                   ctx->fill.part, ctx->fill.count, ctx->fcache, ctx->xtw_i,
                   ctx->rowtab_i[0], ctx->rowtab_i[1], ctx->rowtab_i[2]};
   for (void* p : ptrs)

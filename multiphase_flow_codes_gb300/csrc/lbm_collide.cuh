@@ -37,15 +37,42 @@ struct RatesT {
   // [1..15] A_k, [16] B1r, [17] B2r, [18] 1/19
   long long Li[19];
   int Lsh[19];
-  // the factors of the velocity and force terms, for the all-integer core
-  // (fx_core_int): B1t H1 B2t H2 B3 H3 B6 H6 B7 H7 B8 H8 B9 H9 B10 H10 0.1 0.05
-  long long Ni[18];
-  int Nsh[18];
-  // the same factors at the one scale 2^62 (|c| < 2), so that every product
-  // of the integer core shifts by a compile-time amount: [0..18] as Li,
-  // [19..36] as Ni
-  long long Ci[37];
+  // the same factors and those of the velocity and force terms for the
+  // all-integer core (fx_core_int), each at the scale 2^kFxSc[i] as
+  // Ch * 2^32 + Cl with a signed low word (|Cl| <= 2^31): [0..18] as Li,
+  // [19..36] B1t H1 B2t H2 B3 H3 B6 H6 B7 H7 B8 H8 B9 H9 B10 H10 0.1 0.05.
+  // int_ok: every factor fits its scale (any rates in (0, 2) do)
+  int Ch[37], Cl[37];
+  bool int_ok;
 };
+
+constexpr int kFxIn = 58, kFxInMax = -3;    // inputs, forward transform
+constexpr int kFxOut = 61, kFxOutMax = -5;  // scaled moments, inverse transform
+constexpr int kFxF = 70;                    // body forces: |F| < 2^-7 at 2^-70
+constexpr int kFxUU = 64;                   // velocities and u_a u_b inside fx_core_int
+
+// Scale 2^-kFxM(k) of the scaled moment k in the integer core: kFxOut, but
+// finer for the two that the inverse transform multiplies by up to 30 and 12.
+__host__ __device__ constexpr int kFxM(int k) { return k == 1 ? 63 : (k == 2 ? 62 : kFxOut); }
+// The integer core sums the products of a moment at the scale
+// 2^-(kFxM(k) + kFxS(k)) and rounds the sum once, by a shift of kFxS(k).  64
+// takes the high word as it is; the moments whose factor on the populations
+// is larger than 2^-4 (|A_k| <= c_k: 1/12 for 8, 1/4 for 10..12, 1/8 for
+// 13..15) need a smaller one so that the factor fits 63 bits.
+__host__ __device__ constexpr int kFxS(int k) {
+  return k == 8 || k >= 13 ? 63 : (k >= 10 ? 62 : 64);
+}
+// scale of factor i of RatesT::Ch: that of its moment's sum over that of the
+// value it multiplies
+__host__ __device__ constexpr int kFxSc(int i) {
+  if (i <= 15) return kFxM(i) + kFxS(i) - kFxIn;              // A_k ev_k
+  if (i <= 18) return kFxM(i - 15) + kFxS(i - 15) - kFxIn;    // B1r, B2r, 1/19 times rho
+  // velocity terms at 2^-kFxUU (even), force terms at 2^-kFxF (odd); the
+  // momentum's last two at the scales of moment 3
+  const int n = i - 19, sv = (n & 1) ? kFxF : kFxUU;
+  const int k = n < 2 ? 1 : n < 4 ? 2 : n < 6 ? 3 : n < 14 ? 6 + (n - 6) / 2 : n < 16 ? 10 : 3;
+  return kFxM(k) + kFxS(k) - sv;
+}
 
 // c as (integer m, shift sh) with c = m * 2^-sh exactly and |m| in
 // [2^61, 2^62) (m = 0, sh = 64 for c = 0)
@@ -84,13 +111,18 @@ RatesT<T> rates_t(const Rates& r) {
                          -2.0 / 3.0 * Bk(3), -2.0 / 3.0 * Hk(3), Bk(6), 2.0 * Hk(6),
                          r.omegxx * Bk(7), -Hk(7), Bk(8), 2.0 * Hk(8), r.omegxx * Bk(9), -Hk(9),
                          Bk(10), Hk(10), 0.1, 0.05};
-  for (int k = 0; k < 18; ++k) fixed_factor(nf[k], &o.Ni[k], &o.Nsh[k]);
-  auto c62 = [](double c) { return (long long)std::llround(std::ldexp(c, 62)); };
-  for (int k = 0; k < 16; ++k) o.Ci[k] = c62(ck[k] * (1.0 - sk[k]));
-  o.Ci[16] = c62(-11.0 * Bk(1));
-  o.Ci[17] = c62(r.omegepsl * Bk(2));
-  o.Ci[18] = c62(1.0 / 19.0);
-  for (int k = 0; k < 18; ++k) o.Ci[19 + k] = c62(nf[k]);
+  o.int_ok = true;
+  for (int i = 0; i < 37; ++i) {
+    const double c = i < 16 ? ck[i] * (1.0 - sk[i])
+                   : i == 16 ? -11.0 * Bk(1) : i == 17 ? r.omegepsl * Bk(2)
+                   : i == 18 ? 1.0 / 19.0 : nf[i - 19];
+    const double v = std::ldexp(c, kFxSc(i));
+    const bool fits = std::fabs(v) < 9.2e18;  // below 2^63 - 2^31
+    o.int_ok = o.int_ok && fits;
+    const long long m = fits ? (long long)std::llround(v) : 0;
+    o.Cl[i] = (int)(unsigned)(unsigned long long)m;
+    o.Ch[i] = (int)((m - o.Cl[i]) >> 32);
+  }
   return o;
 }
 
@@ -258,8 +290,7 @@ __host__ __device__ __forceinline__ void collide_fast(T (&f)[NPOP], T fpx, T fpy
 // by a false return with f untouched; the caller then collides it with
 // collide_fast.
 
-constexpr int kFxIn = 58, kFxInMax = -3;    // inputs, forward transform
-constexpr int kFxOut = 61, kFxOutMax = -5;  // scaled moments, inverse transform
+// (kFxIn, kFxInMax; kFxOut, kFxOutMax above)
 // a node whose largest |f| is below 2^kFxMinExp keeps FP64's relative
 // precision through the FP64 path (fixed point resolves 2^-61 absolute)
 constexpr int kFxMinExp = -12;
@@ -314,11 +345,12 @@ __host__ __device__ __forceinline__ long long fx_mul(long long v, long long m, i
   return (long long)(p >> s);
 }
 
-// |x| < 2^(kFxOutMax) at scale 2^-kFxOut
+// |x| < 2^(kFxOutMax) at scale 2^-K
+template <int K = kFxOut>
 __host__ __device__ __forceinline__ unsigned fx_out_of_range(long long x) {
-  // |x| >= 2^(kFxOut + kFxOutMax) = 2^56, on the high word: the bound's low
-  // word is zero, so x + 2^56 >= 2^57 is (hi + 2^24) >= 2^25 in 32 bits
-  constexpr unsigned hlim = 1u << (kFxOut + kFxOutMax - 32);
+  // |x| >= 2^(K + kFxOutMax) (2^56 for kFxOut), on the high word: the bound's
+  // low word is zero, so x + 2^56 >= 2^57 is (hi + 2^24) >= 2^25 in 32 bits
+  constexpr unsigned hlim = 1u << (K + kFxOutMax - 32);
   return ((unsigned)((unsigned long long)x >> 32) + hlim) & ~(2 * hlim - 1);
 }
 
@@ -334,7 +366,6 @@ __host__ __device__ __forceinline__ unsigned fx_out_of_range(long long x) {
 // 2^-kFxOut; false when a moment leaves its range.  The previous step's body
 // force fp (the velocity's F/2) is FP64, or (FP = long long) fixed point at
 // 2^-kFxF, added to the momentum sums exactly.
-constexpr int kFxF = 70;  // body forces in fixed point: |F| < 2^-7 at 2^-70
 template <typename FP>
 __host__ __device__ __forceinline__ bool fx_core(const long long (&g)[NPOP], FP fpx, FP fpy,
                                                  FP fpz, double fx, double fy, double fz,
@@ -479,24 +510,55 @@ __host__ __device__ __forceinline__ bool fx_core(const long long (&g)[NPOP], FP 
   return true;
 }
 
-// round(a * b * 2^-s), s >= 1: one exact 128-bit product, one rounding.
-// (An explicit carry chain, mad.lo.cc / madc.hi with the rounding constant
-// as the addend, measured 8 % slower for the whole FP64 step than this.)
-__host__ __device__ __forceinline__ long long mul_round(long long a, long long b, int s) {
-  const __int128 p = (__int128)a * (__int128)b + ((__int128)1 << (s - 1));
-  return (long long)(p >> s);
+// A 64-bit fixed-point value as h * 2^32 + l with a signed low word, so that
+// every partial product of two such values is one signed 32 x 32 -> 64 bit
+// multiply-add (|v| < 2^63 - 2^31).
+struct Split { int h, l; };
+__host__ __device__ __forceinline__ Split split(long long v) {
+  const int l = (int)(unsigned)(unsigned long long)v;
+  return {(int)(v >> 32) + (int)((unsigned)l >> 31), l};
+}
+
+// (sum of n products a_i b_i) / 2^S, rounded to nearest once: the terms at
+// 2^64 and 2^32 exactly, the products of the low words left out.  Those are
+// below 2^62 each: a quarter of a unit of the result for S = 64, with zero
+// mean, less than the rounding of every product by itself.
+// Three multiply-adds a product (a 128-bit product lowered by the compiler
+// takes about twenty instructions): k_fused_fixed, bound by integer issue
+// with the exact products, ran 2354 instructions a node with them.
+template <int S, int n>
+__host__ __device__ __forceinline__ long long dot_shift(const Split (&a)[n], const Split (&b)[n]) {
+  static_assert(S > 32 && S <= 64, "shift");
+  long long q = 1LL << (S - 33);
+#pragma unroll
+  for (int i = 0; i < n; ++i) {
+    q += (long long)a[i].h * b[i].l;
+    q += (long long)a[i].l * b[i].h;
+  }
+  long long p = q >> 32;
+#pragma unroll
+  for (int i = 0; i < n; ++i) p += (long long)a[i].h * b[i].h;
+  if (S == 64) return p;
+  const unsigned ql = (unsigned)(unsigned long long)q;
+#ifdef __CUDA_ARCH__
+  const unsigned pl = (unsigned)(unsigned long long)p, ph = (unsigned)((unsigned long long)p >> 32);
+  const unsigned rl = __funnelshift_l(ql, pl, 64 - S), rh = __funnelshift_l(pl, ph, 64 - S);
+  return (long long)(((unsigned long long)rh << 32) | rl);
+#else
+  return (long long)(((unsigned long long)p << ((64 - S) & 63)) | (ql >> ((S - 32) & 31)));
+#endif
 }
 
 // fx_core with the velocity and force terms as integer products too, so the
-// collision issues no FP64 instruction: the velocity u (scale 2^-kFxIn) and
-// this step's body force F (2^-kFxF) enter as integers; the products
-// u_a u_b are rounded once to 2^-64 and F_a u_b to 2^-kFxF; each term of a
-// moment is one exact 128-bit product of such a value and a fixed-point
-// factor (RatesT::Ni), rounded once to 2^-kFxOut.  Ranges, so that nothing
+// collision issues no FP64 instruction: the velocity u (scale 2^-kFxIn, then
+// 2^-kFxUU) and this step's body force F (2^-kFxF) enter as integers; the
+// products u_a u_b are rounded once to 2^-kFxUU and F_a u_b to 2^-kFxF, and
+// each moment is one sum of products of such values and fixed-point factors
+// (RatesT::Ch), rounded once to 2^-kFxOut.  Ranges, so that nothing
 // overflows: |u| < 2^-2 and |F| < 2^-9 (a node beyond them is declined, as
-// is one whose moments leave their ranges).  The roundings (2^-62 per term)
-// are those of fx_core's conversions from FP64.
-constexpr int kFxUU = 64;  // u_a u_b
+// is one whose moments leave their ranges).  With |g| < 2^55 the largest sum
+// of middle terms is M1's: below 8.6e18 (the linear program over all inputs
+// with |u_a| < 2^-2, and low words of 2^31) against 2^63 = 9.2e18.
 //
 // bias is added to every output (through tl1, which each of them holds once):
 // the caller's rounding constant costs one add instead of nineteen.
@@ -521,8 +583,8 @@ __host__ __device__ __forceinline__ bool fx_core_int(const long long (&g)[NPOP],
   const I sum3 = D1 + D2;
   const I A = s78 - s910, Bv = d1516 + d1718;
   const I sum4 = A + Bv;
-  const I C = s1112 - s1314, Dd = s1516 - s1718;
-  const I sum5 = C + Dd;
+  const I C1 = s1112 - s1314, Dd = s1516 - s1718;
+  const I sum5 = C1 + Dd;
   const I sum7 = a3 + a5, sum8 = Sxy + Sxz, sum10 = a3 - a5, sum11 = Sxy - Sxz;
   const I rho = g[0] + sum1 + sum2;
   const I ev1 = -30 * g[0] - 11 * sum1 + 8 * sum2;
@@ -550,53 +612,85 @@ __host__ __device__ __forceinline__ bool fx_core_int(const long long (&g)[NPOP],
     const unsigned badf = ((hw(Fx) + flim) | (hw(Fy) + flim) | (hw(Fz) + flim)) & ~(2 * flim - 1);
     if (bad | badf) return false;
   }
-  // products (collision.f90:66-81): u_a u_b at 2^-64, F_a u_b at 2^-kFxF
-  constexpr int suu = 2 * kFxIn - kFxUU, sfu = kFxIn;
-  const I qxx = mul_round(ux, ux, suu), qyy = mul_round(uy, uy, suu), qzz = mul_round(uz, uz, suu);
-  const I qxy = mul_round(ux, uy, suu), qyz = mul_round(uy, uz, suu), qxz = mul_round(ux, uz, suu);
-  const I pa = mul_round(Fx, ux, sfu), pb = mul_round(Fy, uy, sfu), pc = mul_round(Fz, uz, sfu);
-  const I t1 = qxx + qyy + qzz;
-  const I eq6 = 2 * qxx - qyy - qzz, eq8 = qyy - qzz;
-  const I G3 = pa + pb + pc, e6 = 2 * pa - pb - pc, e8 = pb - pc;
-  const I m10 = mul_round(Fx, uy, sfu) + mul_round(Fy, ux, sfu);
-  const I m11 = mul_round(Fy, uz, sfu) + mul_round(Fz, uy, sfu);
-  const I m12 = mul_round(Fx, uz, sfu) + mul_round(Fz, ux, sfu);
-  // factor k (at 2^-62) times a value at scale 2^-sv, at 2^-kFxOut: the
-  // shifts are compile-time constants
-  auto N = [&](int k, I v, int sv) { return mul_round(v, r.Ci[19 + k], 62 + sv - kFxOut); };
-  auto L = [&](int k, I v) { return mul_round(v, r.Ci[k], 62 + kFxIn - kFxOut); };
+  // products (collision.f90:66-81): u_a u_b at 2^-kFxUU, F_a u_b at 2^-kFxF
+  constexpr int su = kFxUU - kFxIn;
+  static_assert(kFxUU == 64, "products by their high words");
+  const Split U[3] = {split(ux << su), split(uy << su), split(uz << su)};
+  const Split G[3] = {split(Fx), split(Fy), split(Fz)};
+  auto mul = [](Split a, Split b) {
+    const Split x[1] = {a}, y[1] = {b};
+    return dot_shift<64, 1>(x, y);
+  };
+  auto mul2 = [](Split a, Split b, Split c, Split d) {
+    const Split x[2] = {a, c}, y[2] = {b, d};
+    return dot_shift<64, 2>(x, y);
+  };
+  const I qxx = mul(U[0], U[0]), qyy = mul(U[1], U[1]), qzz = mul(U[2], U[2]);
+  const Split qxy = split(mul(U[0], U[1])), qyz = split(mul(U[1], U[2])), qxz = split(mul(U[0], U[2]));
+  const I pa = mul(G[0], U[0]), pb = mul(G[1], U[1]), pc = mul(G[2], U[2]);
+  const Split t1 = split(qxx + qyy + qzz);
+  const Split eq6 = split(2 * qxx - qyy - qzz), eq8 = split(qyy - qzz);
+  const Split G3 = split(pa + pb + pc), e6 = split(2 * pa - pb - pc), e8 = split(pb - pc);
+  const Split m10 = split(mul2(G[0], U[1], G[1], U[0]));
+  const Split m11 = split(mul2(G[1], U[2], G[2], U[1]));
+  const Split m12 = split(mul2(G[0], U[2], G[2], U[0]));
+  const Split rhos = split(rho);
+  auto C = [&](int i) { return Split{r.Ch[i], r.Cl[i]}; };
+  auto N = [&](int k) { return C(19 + k); };
   I M[16];
-  M[1] = L(1, ev1) + L(16, rho) + N(0, t1, kFxUU) + N(1, G3, kFxF);
-  M[2] = L(2, ev2) + L(17, rho) + N(2, t1, kFxUU) + N(3, G3, kFxF);
-  M[3] = L(3, ev3) + N(4, ux, kFxIn) + N(5, Fx, kFxF);
-  M[4] = L(4, ev4) + N(4, uy, kFxIn) + N(5, Fy, kFxF);
-  M[5] = L(5, ev5) + N(4, uz, kFxIn) + N(5, Fz, kFxF);
-  M[6] = L(6, ev6) + N(6, eq6, kFxUU) + N(7, e6, kFxF);
-  M[7] = L(7, ev7) + N(8, eq6, kFxUU) + N(9, e6, kFxF);
-  M[8] = L(8, ev8) + N(10, eq8, kFxUU) + N(11, e8, kFxF);
-  M[9] = L(9, ev9) + N(12, eq8, kFxUU) + N(13, e8, kFxF);
-  M[10] = L(10, d78 - d910) + N(14, qxy, kFxUU) + N(15, m10, kFxF);
-  M[11] = L(11, d1516 - d1718) + N(14, qyz, kFxUU) + N(15, m11, kFxF);
-  M[12] = L(12, d1112 - d1314) + N(14, qxz, kFxUU) + N(15, m12, kFxF);
-  M[13] = L(13, D1 - D2);
-  M[14] = L(14, Bv - A);
-  M[15] = L(15, C - Dd);
-  const I tl1 = L(18, rho);
-  const I tl6 = N(16, ux, kFxIn) + N(17, Fx, kFxF);
-  const I tl8 = N(16, uy, kFxIn) + N(17, Fy, kFxF);
-  const I tl10 = N(16, uz, kFxIn) + N(17, Fz, kFxF);
-  unsigned out = 0;
+  // a moment of the populations, a velocity term and a force term
+  auto moment = [&](auto S, int k, I ev, Split v, int nv, Split w, int nw) {
+    const Split x[3] = {split(ev), v, w}, y[3] = {C(k), N(nv), N(nw)};
+    return dot_shift<decltype(S)::value, 3>(x, y);
+  };
+  // moments 1 and 2 also hold a density term
+  auto moment_rho = [&](int k, I ev, Split v, int nv, Split w, int nw) {
+    const Split x[4] = {split(ev), rhos, v, w}, y[4] = {C(k), C(15 + k), N(nv), N(nw)};
+    return dot_shift<kFxS(1), 4>(x, y);
+  };
+  auto alone = [&](int k, I ev) {
+    const Split x[1] = {split(ev)}, y[1] = {C(k)};
+    return dot_shift<kFxS(13), 1>(x, y);
+  };
+  auto momentum = [&](int a) {
+    const Split x[2] = {U[a], G[a]}, y[2] = {N(16), N(17)};
+    return dot_shift<64, 2>(x, y);
+  };
+  const std::integral_constant<int, kFxS(3)> s64{};
+  const std::integral_constant<int, kFxS(8)> s8{};
+  const std::integral_constant<int, kFxS(10)> s10{};
+  M[1] = moment_rho(1, ev1, t1, 0, G3, 1);
+  M[2] = moment_rho(2, ev2, t1, 2, G3, 3);
+  M[3] = moment(s64, 3, ev3, U[0], 4, G[0], 5);
+  M[4] = moment(s64, 4, ev4, U[1], 4, G[1], 5);
+  M[5] = moment(s64, 5, ev5, U[2], 4, G[2], 5);
+  M[6] = moment(s64, 6, ev6, eq6, 6, e6, 7);
+  M[7] = moment(s64, 7, ev7, eq6, 8, e6, 9);
+  M[8] = moment(s8, 8, ev8, eq8, 10, e8, 11);
+  M[9] = moment(s64, 9, ev9, eq8, 12, e8, 13);
+  M[10] = moment(s10, 10, d78 - d910, qxy, 14, m10, 15);
+  M[11] = moment(s10, 11, d1516 - d1718, qyz, 14, m11, 15);
+  M[12] = moment(s10, 12, d1112 - d1314, qxz, 14, m12, 15);
+  M[13] = alone(13, D1 - D2);
+  M[14] = alone(14, Bv - A);
+  M[15] = alone(15, C1 - Dd);
+  const Split xr[1] = {rhos}, yr[1] = {C(18)};
+  const I tl1 = dot_shift<64, 1>(xr, yr);
+  const I tl6 = momentum(0), tl8 = momentum(1), tl10 = momentum(2);
+  unsigned out = fx_out_of_range<kFxM(1)>(M[1]) | fx_out_of_range<kFxM(2)>(M[2]);
 #pragma unroll
-  for (int k = 1; k < 16; ++k) out |= fx_out_of_range(M[k]);
+  for (int k = 3; k < 16; ++k) out |= fx_out_of_range(M[k]);
   out |= fx_out_of_range(tl1) | fx_out_of_range(tl6) | fx_out_of_range(tl8) |
          fx_out_of_range(tl10);
   if (out) return false;
 
-  // inverse transform, exact (collision.f90:160-200)
+  // inverse transform (collision.f90:160-200): exact but for the one rounding
+  // from the finer scales of M1 and M2 of the three sums that hold them
+  static_assert(kFxM(1) == kFxOut + 2 && kFxM(2) == kFxOut + 1, "shifts below");
   const I tlb = tl1 + bias;
-  h[0] = tlb - 30 * M[1] + 12 * M[2];
-  const I suma = tlb - 11 * M[1] - 4 * M[2];
-  const I sumb = tlb + 8 * M[1] + M[2];
+  h[0] = (4 * tlb - 30 * M[1] + 24 * M[2]) >> 2;
+  const I suma = tlb + ((2 - 11 * M[1] - 8 * M[2]) >> 2);
+  const I sumb = tlb + 2 * M[1] + ((M[2] + 1) >> 1);
   const I sumc = tl6 - 4 * M[3];
   const I sumd = 2 * M[6] - 4 * M[7];
   const I sume = tl8 - 4 * M[4];

@@ -350,13 +350,13 @@ __device__ __forceinline__ void body_force_fxd(const ForceView<double>& fv, cons
 // once, body_force_fxd; otherwise exact integer products, body_force_fx): the
 // previous step's enters the velocity as an exact integer add; the force
 // cache (fcache_mode as in k_fused) holds them as 64-bit integers at 2^-kFxF.
-// CTAs of 128 threads per SM: four with the integer core (128 registers;
-// with the force series on the FP64 pipe 3.4 % faster at 256^3 than five at
-// 96 registers, twice the spills, and 2.6 % faster than three at 168, no
-// spills); five with the FP64-product core (96 registers, 3 % faster than
-// four there).
+// Five CTAs of 128 threads per SM (96 registers): the integer core is now
+// short enough that loads and stores bound it, and more warps hide them
+// (256^3 with 1000 spheres: 1.01 ms, 5.0 TB/s of populations; four CTAs at
+// 128 registers 1.11 ms, three 1.24 ms, six 1.02 ms; before, with 128-bit
+// products, 1.54 ms at four).
 template <bool CHANNEL, bool INTCORE>
-__global__ void __launch_bounds__(128, INTCORE ? 4 : 5) k_fused_fixed(Geometry g, RatesT<double> r,
+__global__ void __launch_bounds__(128, 5) k_fused_fixed(Geometry g, RatesT<double> r,
                                                          const long long* __restrict__ fin,
                                                          long long* __restrict__ fout,
                                                          const int32_t* __restrict__ isnodes,
@@ -859,7 +859,7 @@ void launch_fused_fixed(const Geometry& g, const Rates& r, bool int_core, const 
   auto launch = [&](auto kern) {
     kern<<<row_grid(g, B), B, 0, s>>>(g, rt, gi, go, isnodes, fprev, fnew, fci, fcache_mode, st);
   };
-  if (int_core)
+  if (int_core && rt.int_ok)
     g.channel ? launch(k_fused_fixed<true, true>) : launch(k_fused_fixed<false, true>);
   else
     g.channel ? launch(k_fused_fixed<true, false>) : launch(k_fused_fixed<false, false>);

@@ -318,8 +318,14 @@ struct LinkSlab {
   int cap;
   void* sweeps;      // per particle: nearest-image sweep events of the 3 axes (kSweepBytes)
   int32_t* sweep_ok; // per particle and axis: 1 if the sweep reached its fixed point
+  // a particle's bounce-back over several blocks (k_bounce): FP64, their
+  // partial force and torque sums (6 per block, kBounceSplit blocks); the
+  // count of blocks done, zero between launches
+  double* bsum;
+  int32_t* bdone;
 };
 constexpr int kSweepBytes = 7 * 96;
+constexpr int kBounceSplit = 24;
 // alpha_fp32: link fractions in single precision (the FP32 population path)
 void launch_links(const Geometry& g, const ParticleView& pv, int32_t* isnodes,
                   LinkSlab ls, DevStatus* st, int alpha_fp32, cudaStream_t s,

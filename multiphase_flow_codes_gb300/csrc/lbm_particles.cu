@@ -14,6 +14,8 @@
 //   k_move         beads_move (2295-2394)       one thread per particle
 //   k_wrap / k_overlap  beads_redistribute's wrap and overlap check
 //   k_filling      beads_filling (2793-3111)    refill of uncovered nodes
+#include <algorithm>
+
 #include <cub/block/block_reduce.cuh>
 #include <cub/block/block_scan.cuh>
 
@@ -702,21 +704,29 @@ __device__ __forceinline__ T read_post(const Geometry& g, const T* f, int pushed
   return ld_pop(g, f, q * N + it + g.nx * (jt + g.ny * kt));
 }
 
-// threads per particle block of the bounce-back: 128 threads leave fewer
-// idle lanes in the last pass over a particle's ~1000 links than 256, and
-// eight such blocks fit an SM (the batched kernel uses the same count, so a
-// box's force sums run in the same order alone and in a batch)
+// threads per block of the bounce-back: small blocks leave fewer idle lanes in
+// the last pass over a particle's ~1000 links (1000 spheres at 256^3, FP32:
+// 256 threads 75 us, 128 threads 72 us); FP64, two blocks of 64 threads a
+// sphere take the same time as one of 128 (137 and 136 us) and split finer
 template <typename T>
-constexpr int bounce_threads() { return 128; }
+constexpr int bounce_threads() { return sizeof(T) == 8 ? 64 : 128; }
+template <typename T>
+constexpr int bounce_blocks() { return 1024 / bounce_threads<T>(); }  // resident per SM
 
-// beads_collision for one particle per block of NT threads: every link
-// computes the bounced population f9 (stored per link) and its momentum
-// exchange.
+// beads_collision: every link computes the bounced population f9 (stored
+// per link) and its momentum exchange.  `split` blocks of NT threads share a
+// particle's links (FP64; FP32 blocks are one per particle, so that a box's
+// compensated sums run in the same order alone and in a batch).  A pass of NT
+// links costs one chain of dependent loads and FP64 operations, about 7 us,
+// whatever the number of blocks, so with few particles one block each leaves
+// the GPU idle for some ten passes: 64^3 with 16 spheres took 84 us, split in
+// eleven 17 us.  The block that finishes last adds the partial sums in block
+// order.
 template <typename T, int NT>
-__device__ __forceinline__ void k_bounce_body(int bx, int gx, Geometry g, ParticleView pv, const T* f, int pushed,
+__device__ __forceinline__ void k_bounce_body(int bx, int split, Geometry g, ParticleView pv, const T* f, int pushed,
                                                const int32_t* __restrict__ isnodes, LinkSlab ls,
                                                double* fHIp, double* torqp) {
-  const int p = bx;
+  const int p = bx / split, part_id = bx - p * split;
   if (p >= pv.npart) return;
   const int cnt = ls.count[p];
   const int32_t* code = ls.code + (long long)p * ls.cap;
@@ -725,8 +735,7 @@ __device__ __forceinline__ void k_bounce_body(int bx, int gx, Geometry g, Partic
   const T* alph = reinterpret_cast<const T*>(ls.alpha + (long long)p * ls.cap);
   T* f9s = reinterpret_cast<T*>(ls.f9 + (long long)p * ls.cap);
   // per-link arithmetic in the population precision R (FP64 plain path,
-  // FP32 shifted path); each thread's partial force/torque sums are
-  // compensated (FP32) or plain FP64, the block sums are FP64
+  // FP32 shifted path)
   using R = T;
   Acc<T> acc6[6];
   // the particle's velocities in the arithmetic precision and the first
@@ -800,7 +809,20 @@ __device__ __forceinline__ void k_bounce_body(int bx, int gx, Geometry g, Partic
     const R v = flip_if(cc < 0, dc);
     return cb == 0 ? flip_if(true, v) : u - v;
   };
-  for (int l = threadIdx.x; l < cnt; l += NT) {
+  // The reference's lever arm is r = d + alpha c (the boundary point);
+  // every quantity it enters is a product with c: the wall velocity
+  // c . (w + omega x r) = c . w + omega . (r x c) and the torque
+  // dff (r x c), and r x c = d x c.  So the per-link arithmetic needs only
+  // e = d x c, which for c in {-1, 0, 1}^3 is selects and one add.
+  auto lever = [&](int i, int j, int k, int ix, int iy, int iz, R& ex, R& ey, R& ez) {
+    const R dx = delta(0, i, xc0, g.nx, g.nxh, !channel);
+    const R dy = delta(1, j, yc0, g.ny, g.nyh, true);
+    const R dz = delta(2, k, zc0, g.nz, g.nzh, true);
+    ex = cross(iz, dy, iy, dz);
+    ey = cross(ix, dz, iz, dx);
+    ez = cross(iy, dx, ix, dy);
+  };
+  for (int l = part_id * NT + threadIdx.x; l < cnt; l += split * NT) {
     // 32-bit decode: node < 2^26
     const int cd = code[l];
     const int ipop = cd & 31;
@@ -822,17 +844,8 @@ __device__ __forceinline__ void k_bounce_body(int bx, int gx, Geometry g, Partic
       im1 = wrapi(im1, g.nx);
       im2 = wrapi(im2, g.nx);
     }
-    // The reference's lever arm is r = d + alpha c (the boundary point);
-    // every quantity it enters is a product with c: the wall velocity
-    // c . (w + omega x r) = c . w + omega . (r x c) and the torque
-    // dff (r x c), and r x c = d x c.  So the per-link arithmetic needs only
-    // e = d x c, which for c in {-1, 0, 1}^3 is selects and one add.
-    const R dx = delta(0, i, xc0, g.nx, g.nxh, !channel);
-    const R dy = delta(1, j, yc0, g.ny, g.nyh, true);
-    const R dz = delta(2, k, zc0, g.nz, g.nzh, true);
-    const R ex = cross(iz, dy, iy, dz);
-    const R ey = cross(ix, dz, iz, dx);
-    const R ez = cross(iy, dx, ix, dy);
+    R ex, ey, ez;
+    lever(i, j, k, ix, iy, iz, ex, ey, ez);
     const R uwpro = fma_r(omg1, ex, fma_r(omg2, ey, fma_r(omg3, ez, tcw[ipop])));
     const R ff1 = R(read_post(g, f, pushed, ipop, i, j, k));
     // The five interpolation cases of beads_collision (B/partlib.f90:1439-1536)
@@ -927,10 +940,14 @@ __device__ __forceinline__ void k_bounce_body(int bx, int gx, Geometry g, Partic
     // component adds NT / 32 of them a lane, then the lanes by an xor
     // butterfly (a fixed order: deterministic)
     __shared__ double part[6][NT];
+    auto put = [&](int c, double v) {
+      if (c < 3) fHIp[3 * p + c] = v; else torqp[3 * p + c - 3] = v;
+    };
 #pragma unroll
     for (int c = 0; c < 6; ++c) part[c][threadIdx.x] = acc6[c].value();
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double* mine = ls.bsum + ((size_t)p * kBounceSplit + part_id) * 6;
     for (int c = warp; c < 6; c += NT / 32) {
       double s = part[c][lane];
 #pragma unroll
@@ -938,18 +955,34 @@ __device__ __forceinline__ void k_bounce_body(int bx, int gx, Geometry g, Partic
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
       if (lane == 0) {
-        if (c < 3) fHIp[3 * p + c] = s; else torqp[3 * p + c - 3] = s;
+        if (split == 1) put(c, s); else mine[c] = s;
       }
+    }
+    if (split == 1) return;
+    __shared__ int s_last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      s_last = atomicAdd(&ls.bdone[p], 1) == split - 1;
+      if (s_last) ls.bdone[p] = 0;
+    }
+    __syncthreads();
+    if (s_last && threadIdx.x < 6) {
+      __threadfence();
+      const double* all = ls.bsum + (size_t)p * kBounceSplit * 6 + threadIdx.x;
+      double s = __ldcg(all);
+      for (int k = 1; k < split; ++k) s += __ldcg(all + 6 * k);
+      put(threadIdx.x, s);
     }
   }
 }
 template <typename T>
-// (64 registers: eight 128-thread blocks per SM, so that the 1000 particle
-// blocks of the workload take one wave)
-__global__ void __launch_bounds__(bounce_threads<T>(), 8) k_bounce(Geometry g, ParticleView pv, const T* f, int pushed,
+// (64 registers: 1024 threads per SM, so that the 1000 spheres of the
+// workload take one wave)
+__global__ void __launch_bounds__(bounce_threads<T>(), bounce_blocks<T>()) k_bounce(Geometry g, ParticleView pv, const T* f, int pushed,
                                                const int32_t* __restrict__ isnodes, LinkSlab ls,
-                                               double* fHIp, double* torqp) {
-  k_bounce_body<T, bounce_threads<T>()>(blockIdx.x, gridDim.x, g, pv, f, pushed, isnodes, ls, fHIp, torqp);
+                                               double* fHIp, double* torqp, int split) {
+  k_bounce_body<T, bounce_threads<T>()>(blockIdx.x, split, g, pv, f, pushed, isnodes, ls, fHIp, torqp);
 }
 
 // the bounce-back stores of beads_collision: f(ipp, x + c) = f9
@@ -1522,12 +1555,24 @@ void launch_links(const Geometry& g, const ParticleView& pv, int32_t* isnodes, L
   { k_links<<<pv.npart, PB, 0, s>>>(g, pv, isnodes, ls, st, alpha_fp32); count_launch(); }
 }
 
+// Blocks that share a particle's bounce-back (FP64): as many as take one
+// wave together, but none beyond the links of a sphere of this radius (about
+// 72 R^2: 18 directions on the surface nodes) and kBounceSplit.
+template <typename T>
+int bounce_split(double rad, long long npart) {
+  if (sizeof(T) == 4) return 1;
+  const long long slots = (long long)bounce_blocks<T>() * sm_count();
+  const int most = (int)std::min<double>(kBounceSplit, std::max(1.0, 72.0 * rad * rad / bounce_threads<T>()));
+  return (int)std::min<long long>(most, std::max<long long>(1, slots / std::max(1LL, npart)));
+}
+
 template <typename T>
 void launch_bounce_back(const Geometry& g, const ParticleView& pv, const T* f, int pushed,
                         const int32_t* isnodes, LinkSlab ls, double* fHIp, double* torqp,
                         cudaStream_t s) {
   if (pv.npart <= 0) return;
-  { k_bounce<T><<<pv.npart, bounce_threads<T>(), 0, s>>>(g, pv, f, pushed, isnodes, ls, fHIp, torqp); count_launch(); }
+  const int split = bounce_split<T>(pv.rad, pv.npart);
+  { k_bounce<T><<<pv.npart * split, bounce_threads<T>(), 0, s>>>(g, pv, f, pushed, isnodes, ls, fHIp, torqp, split); count_launch(); }
 }
 
 template <typename T>
@@ -1603,9 +1648,9 @@ namespace {
   const int nblk = (nblocks_expr);                   \
   if ((int)blockIdx.x >= nblk) return;
 
-__global__ void __launch_bounds__(bounce_threads<float>(), 8) k_bounce_multi(const BoxParticles* boxes) {
+__global__ void __launch_bounds__(bounce_threads<float>(), bounce_blocks<float>()) k_bounce_multi(const BoxParticles* boxes) {
   BOX_OR_RETURN(B.pv.npart)
-  k_bounce_body<float, bounce_threads<float>()>(blockIdx.x, nblk, B.g, B.pv, B.f, 1, B.flags_cur, B.ls,
+  k_bounce_body<float, bounce_threads<float>()>(blockIdx.x, 1, B.g, B.pv, B.f, 1, B.flags_cur, B.ls,
                                                 B.ms.fHIp, B.ms.torqp);
 }
 __global__ void __launch_bounds__(PB) k_bounce_store_multi(const BoxParticles* boxes) {
