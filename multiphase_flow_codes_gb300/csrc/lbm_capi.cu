@@ -654,7 +654,8 @@ void unfused_step_t(lbm_ctx* c) {
   materialize_macro(c);
   do_forcing(c);
   launch_collision<T>(c->g, c->r, fbuf<T>(c, c->cur), c->flags[c->fcur], fview<T>(c, c->latest),
-                      mbuf<T>(c, 0), mbuf<T>(c, 1), mbuf<T>(c, 2), mbuf<T>(c, 3), c->stream);
+                      mbuf<T>(c, 0), mbuf<T>(c, 1), mbuf<T>(c, 2), mbuf<T>(c, 3),
+                      c->sums != LBM_SUMS_FLOAT, c->stream);
   if (c->particles_on) {
     launch_bounce_back<T>(c->g, pview(c), fbuf<T>(c, c->cur), 0, c->flags[c->fcur], c->links,
                           c->fHIp, c->torqp, c->stream);
@@ -1755,12 +1756,12 @@ int lbm_collision_mrt(lbm_ctx* ctx) {
   if (ctx->f32)
     launch_collision<float>(ctx->g, ctx->r, fbuf<float>(ctx, ctx->cur), ctx->flags[ctx->fcur],
                             fview<float>(ctx, ctx->latest), mbuf<float>(ctx, 0), mbuf<float>(ctx, 1),
-                            mbuf<float>(ctx, 2), mbuf<float>(ctx, 3), ctx->stream);
+                            mbuf<float>(ctx, 2), mbuf<float>(ctx, 3), false, ctx->stream);
   else
     launch_collision<double>(ctx->g, ctx->r, fbuf<double>(ctx, ctx->cur), ctx->flags[ctx->fcur],
                              fview<double>(ctx, ctx->latest), mbuf<double>(ctx, 0),
                              mbuf<double>(ctx, 1), mbuf<double>(ctx, 2), mbuf<double>(ctx, 3),
-                             ctx->stream);
+                             ctx->sums != LBM_SUMS_FLOAT, ctx->stream);
   ctx->macro_derived = false;
   CK(cudaGetLastError());
   return LBM_OK;
@@ -1870,10 +1871,69 @@ int lbm_rhoupdat(lbm_ctx* ctx) {
   return LBM_OK;
 }
 
+// The pre-relaxation loop by k_relax, one pass an iteration.  Iteration k
+// (counter k) is the collision and streaming of pass k and the rhoupdat of
+// pass k + 1; the loop ends after the iteration whose change is within eps or
+// whose counter passes max_iter, and the last rhoupdat comes without a next
+// collision.  Passes are enqueued a chunk ahead of the host's reading of
+// their changes: a pass after the last one finds that out by itself and
+// leaves everything as it is.
+static int prerelax_passes(lbm_ctx* ctx, double eps, int max_iter, int* iters, double* err) {
+  constexpr int kChunk = 16;
+  unsigned long long* change = reinterpret_cast<unsigned long long*>(ctx->partial);  // [kChunk + 1]
+  unsigned long long* host = reinterpret_cast<unsigned long long*>(ctx->partial_host);
+  // pass p reads buffer in(p): the populations after p iterations
+  const int b0 = ctx->cur;
+  auto in = [&](int p) { return (b0 + p) & 1; };
+  auto pass = [&](int p, const unsigned long long* before, unsigned long long* slot) {
+    return launch_relax(ctx->g, ctx->r, fbuf<double>(ctx, in(p)), fbuf<double>(ctx, in(p + 1)),
+                        ctx->flags[ctx->fcur], fview<double>(ctx, ctx->latest), mbuf<double>(ctx, 0),
+                        mbuf<double>(ctx, 1), mbuf<double>(ctx, 2), mbuf<double>(ctx, 3), p == 0,
+                        before, slot, eps, ctx->stream);
+  };
+  if (!pass(0, nullptr, nullptr)) return 1;  // rates outside the integer core's scales
+  const int last = max_iter + 2;             // the pass after the last iteration
+  for (int p = 1;;) {
+    const int n = std::min(kChunk, last - p + 1);
+    CK(cudaMemsetAsync(change, 0, n * sizeof *change, ctx->stream));
+    for (int i = 0; i < n; ++i) {
+      const unsigned long long* before = i ? change + i - 1 : nullptr;
+      if (p + i < last)
+        pass(p + i, before, change + i);
+      else
+        launch_rhoupdat_change(ctx->g, fbuf<double>(ctx, in(p + i)), mbuf<double>(ctx, 0), before,
+                               change + i, eps, ctx->stream);
+    }
+    CK(cudaMemcpyAsync(host, change, n * sizeof *change, cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+    for (int i = 0; i < n; ++i) {
+      double e;
+      std::memcpy(&e, &host[i], sizeof e);
+      const int counter = p + i - 1;
+      const bool end = e <= eps || counter > max_iter;
+      if (end || !std::isfinite(e)) {
+        ctx->cur = in(p + i);
+        ctx->macro_derived = false;
+        if (!std::isfinite(e))
+          return fail(ctx, LBM_ERR_NONFINITE, "pre-relaxation: density not finite");
+        if (iters) *iters = counter;
+        if (err) *err = e;
+        return LBM_OK;
+      }
+    }
+    p += n;
+  }
+}
+
 int lbm_prerelax(lbm_ctx* ctx, double eps, int max_iter, int* iters, double* err) {
   if (!ctx || !(eps >= 0.0) || max_iter < 0) return LBM_ERR_ARG;
   if (ctx->in_batch) return fail(ctx, LBM_ERR_STATE, "a batched context steps only through its batch");
   materialize_macro(ctx);
+  // (max_iter + 2 must not overflow; such a count takes the loop below)
+  if (!ctx->f32 && ctx->sums != LBM_SUMS_FLOAT && max_iter < (1 << 30)) {
+    const int rc = prerelax_passes(ctx, eps, max_iter, iters, err);
+    if (rc <= 0) return rc;
+  }
   unsigned long long* maxbits = reinterpret_cast<unsigned long long*>(ctx->partial);
   int istep = 0;
   double e = 0.0;

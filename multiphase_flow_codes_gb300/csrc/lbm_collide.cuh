@@ -298,12 +298,15 @@ constexpr int kFxMinExp = -12;
 // x -> round(x * 2^K) (half away from zero); emax collects the largest
 // biased exponent seen (the caller tests the range once for all values).
 // Values below 2^(-K-1) (zero, subnormals) give 0.
-template <int K>
-__host__ __device__ __forceinline__ long long fx_from(double x, int& emax) {
+__host__ __device__ __forceinline__ int fx_exponent(double x) {  // biased
+  unsigned long long b;
+  memcpy(&b, &x, 8);
+  return (int)(b >> 52) & 0x7ff;
+}
+__host__ __device__ __forceinline__ long long fx_from_k(double x, int K) {
   unsigned long long b;
   memcpy(&b, &x, 8);
   const int e = (int)(b >> 52) & 0x7ff;
-  emax = emax > e ? emax : e;
   // magnitude with the hidden bit at bit 63: |x| = m * 2^(e - 1086)
   const unsigned long long m = (b << 11) | 0x8000000000000000ULL;
   // |x| * 2^K = m * 2^-(1086 - K - e): shift by one less, add the half, shift
@@ -312,10 +315,15 @@ __host__ __device__ __forceinline__ long long fx_from(double x, int& emax) {
   const long long sg = (long long)b >> 63;  // 0 or -1
   return ((long long)v ^ sg) - sg;
 }
+template <int K>
+__host__ __device__ __forceinline__ long long fx_from(double x, int& emax) {
+  const int e = fx_exponent(x);
+  emax = emax > e ? emax : e;
+  return fx_from_k(x, K);
+}
 
 // v * 2^-K as a double, rounded to nearest (ties away from zero)
-template <int K>
-__host__ __device__ __forceinline__ double fx_to(long long v) {
+__host__ __device__ __forceinline__ double fx_to_k(long long v, int K) {
   const long long sg = v >> 63;
   unsigned long long a = (unsigned long long)((v ^ sg) - sg);
 #ifdef __CUDA_ARCH__
@@ -334,6 +342,8 @@ __host__ __device__ __forceinline__ double fx_to(long long v) {
   memcpy(&d, &bits, 8);
   return a ? d : 0.0;
 }
+template <int K>
+__host__ __device__ __forceinline__ double fx_to(long long v) { return fx_to_k(v, K); }
 
 
 // round(v * m * 2^-sh_total) with v a fixed-point value (scale 2^-kFxIn),
@@ -562,11 +572,10 @@ __host__ __device__ __forceinline__ long long dot_shift(const Split (&a)[n], con
 //
 // bias is added to every output (through tl1, which each of them holds once):
 // the caller's rounding constant costs one add instead of nineteen.
-__host__ __device__ __forceinline__ bool fx_core_int(const long long (&g)[NPOP], long long fpx,
-                                                     long long fpy, long long fpz, long long Fx,
-                                                     long long Fy, long long Fz,
-                                                     const RatesT<double>& r,
-                                                     long long (&h)[NPOP], long long bias = 0) {
+// The integer sums of the forward transform (collision.f90:101-118): density,
+// momentum and the moments ev_1..ev_15 of the populations g.
+struct FxSums { long long rho, jx, jy, jz, ev[16]; };
+__host__ __device__ __forceinline__ void fx_sums(const long long (&g)[NPOP], FxSums& o) {
   typedef long long I;
   const I a1 = g[1] + g[2], d1 = g[1] - g[2];
   const I a3 = g[3] + g[4], d3 = g[3] - g[4];
@@ -596,27 +605,33 @@ __host__ __device__ __forceinline__ bool fx_core_int(const long long (&g)[NPOP],
   const I ev7 = -4 * a1 + 2 * (sum7 - Syz) + sum8;
   const I ev8 = sum10 + sum11;
   const I ev9 = -2 * sum10 + sum11;
-  // macrovar: u = sum c f + F_prev / 2, exact at 2^-kFxIn
-  constexpr int sh = kFxF - kFxIn + 1;
-  auto half = [](long long v) { return (v + (1LL << (sh - 1))) >> sh; };
-  const I ux = d1 + sum3 + half(fpx);
-  const I uy = d3 + sum4 + half(fpy);
-  const I uz = d5 + sum5 + half(fpz);
-  {
-    // |u| < 2^-2 and |F| < 2^-9, on the high words (the bounds' low words are
-    // zero, as for the input test of collide_fx_fixed_int)
-    constexpr unsigned ulim = 1u << (kFxIn - 2 - 32);
-    constexpr unsigned flim = 1u << (kFxF - 9 - 32);
-    auto hw = [](long long v) { return (unsigned)((unsigned long long)v >> 32); };
-    const unsigned bad = ((hw(ux) + ulim) | (hw(uy) + ulim) | (hw(uz) + ulim)) & ~(2 * ulim - 1);
-    const unsigned badf = ((hw(Fx) + flim) | (hw(Fy) + flim) | (hw(Fz) + flim)) & ~(2 * flim - 1);
-    if (bad | badf) return false;
-  }
+  o.rho = rho;
+  o.jx = d1 + sum3;
+  o.jy = d3 + sum4;
+  o.jz = d5 + sum5;
+  o.ev[1] = ev1; o.ev[2] = ev2; o.ev[3] = ev3; o.ev[4] = ev4; o.ev[5] = ev5;
+  o.ev[6] = ev6; o.ev[7] = ev7; o.ev[8] = ev8; o.ev[9] = ev9;
+  o.ev[10] = d78 - d910;
+  o.ev[11] = d1516 - d1718;
+  o.ev[12] = d1112 - d1314;
+  o.ev[13] = D1 - D2;
+  o.ev[14] = Bv - A;
+  o.ev[15] = C1 - Dd;
+}
+
+// Relaxation and inverse transform on the sums of one node.  Everything is
+// at the scales of fx_core_int times 2^j: rho (2^-(kFxIn + j)), the velocity U
+// (2^-(kFxUU + j)) and the force Fj (2^-(kFxF + j)); V and F are the velocity
+// and the force at 2^-kFxUU and 2^-kFxF (U and Fj themselves for j = 0), so
+// that the products u_a u_b and F_a u_b are at 2^j times their scales too.
+// False when a moment leaves its range.
+__host__ __device__ __forceinline__ bool fx_relax(const FxSums& o, long long rho, const Split (&U)[3],
+                                                  const Split (&V)[3], const Split (&F)[3],
+                                                  const Split (&Fj)[3], const RatesT<double>& r,
+                                                  long long (&h)[NPOP], long long bias) {
+  typedef long long I;
   // products (collision.f90:66-81): u_a u_b at 2^-kFxUU, F_a u_b at 2^-kFxF
-  constexpr int su = kFxUU - kFxIn;
   static_assert(kFxUU == 64, "products by their high words");
-  const Split U[3] = {split(ux << su), split(uy << su), split(uz << su)};
-  const Split G[3] = {split(Fx), split(Fy), split(Fz)};
   auto mul = [](Split a, Split b) {
     const Split x[1] = {a}, y[1] = {b};
     return dot_shift<64, 1>(x, y);
@@ -625,15 +640,15 @@ __host__ __device__ __forceinline__ bool fx_core_int(const long long (&g)[NPOP],
     const Split x[2] = {a, c}, y[2] = {b, d};
     return dot_shift<64, 2>(x, y);
   };
-  const I qxx = mul(U[0], U[0]), qyy = mul(U[1], U[1]), qzz = mul(U[2], U[2]);
-  const Split qxy = split(mul(U[0], U[1])), qyz = split(mul(U[1], U[2])), qxz = split(mul(U[0], U[2]));
-  const I pa = mul(G[0], U[0]), pb = mul(G[1], U[1]), pc = mul(G[2], U[2]);
+  const I qxx = mul(U[0], V[0]), qyy = mul(U[1], V[1]), qzz = mul(U[2], V[2]);
+  const Split qxy = split(mul(U[0], V[1])), qyz = split(mul(U[1], V[2])), qxz = split(mul(U[0], V[2]));
+  const I pa = mul(F[0], U[0]), pb = mul(F[1], U[1]), pc = mul(F[2], U[2]);
   const Split t1 = split(qxx + qyy + qzz);
   const Split eq6 = split(2 * qxx - qyy - qzz), eq8 = split(qyy - qzz);
   const Split G3 = split(pa + pb + pc), e6 = split(2 * pa - pb - pc), e8 = split(pb - pc);
-  const Split m10 = split(mul2(G[0], U[1], G[1], U[0]));
-  const Split m11 = split(mul2(G[1], U[2], G[2], U[1]));
-  const Split m12 = split(mul2(G[0], U[2], G[2], U[0]));
+  const Split m10 = split(mul2(F[0], U[1], F[1], U[0]));
+  const Split m11 = split(mul2(F[1], U[2], F[2], U[1]));
+  const Split m12 = split(mul2(F[0], U[2], F[2], U[0]));
   const Split rhos = split(rho);
   auto C = [&](int i) { return Split{r.Ch[i], r.Cl[i]}; };
   auto N = [&](int k) { return C(19 + k); };
@@ -653,27 +668,27 @@ __host__ __device__ __forceinline__ bool fx_core_int(const long long (&g)[NPOP],
     return dot_shift<kFxS(13), 1>(x, y);
   };
   auto momentum = [&](int a) {
-    const Split x[2] = {U[a], G[a]}, y[2] = {N(16), N(17)};
+    const Split x[2] = {U[a], Fj[a]}, y[2] = {N(16), N(17)};
     return dot_shift<64, 2>(x, y);
   };
   const std::integral_constant<int, kFxS(3)> s64{};
   const std::integral_constant<int, kFxS(8)> s8{};
   const std::integral_constant<int, kFxS(10)> s10{};
-  M[1] = moment_rho(1, ev1, t1, 0, G3, 1);
-  M[2] = moment_rho(2, ev2, t1, 2, G3, 3);
-  M[3] = moment(s64, 3, ev3, U[0], 4, G[0], 5);
-  M[4] = moment(s64, 4, ev4, U[1], 4, G[1], 5);
-  M[5] = moment(s64, 5, ev5, U[2], 4, G[2], 5);
-  M[6] = moment(s64, 6, ev6, eq6, 6, e6, 7);
-  M[7] = moment(s64, 7, ev7, eq6, 8, e6, 9);
-  M[8] = moment(s8, 8, ev8, eq8, 10, e8, 11);
-  M[9] = moment(s64, 9, ev9, eq8, 12, e8, 13);
-  M[10] = moment(s10, 10, d78 - d910, qxy, 14, m10, 15);
-  M[11] = moment(s10, 11, d1516 - d1718, qyz, 14, m11, 15);
-  M[12] = moment(s10, 12, d1112 - d1314, qxz, 14, m12, 15);
-  M[13] = alone(13, D1 - D2);
-  M[14] = alone(14, Bv - A);
-  M[15] = alone(15, C1 - Dd);
+  M[1] = moment_rho(1, o.ev[1], t1, 0, G3, 1);
+  M[2] = moment_rho(2, o.ev[2], t1, 2, G3, 3);
+  M[3] = moment(s64, 3, o.ev[3], U[0], 4, Fj[0], 5);
+  M[4] = moment(s64, 4, o.ev[4], U[1], 4, Fj[1], 5);
+  M[5] = moment(s64, 5, o.ev[5], U[2], 4, Fj[2], 5);
+  M[6] = moment(s64, 6, o.ev[6], eq6, 6, e6, 7);
+  M[7] = moment(s64, 7, o.ev[7], eq6, 8, e6, 9);
+  M[8] = moment(s8, 8, o.ev[8], eq8, 10, e8, 11);
+  M[9] = moment(s64, 9, o.ev[9], eq8, 12, e8, 13);
+  M[10] = moment(s10, 10, o.ev[10], qxy, 14, m10, 15);
+  M[11] = moment(s10, 11, o.ev[11], qyz, 14, m11, 15);
+  M[12] = moment(s10, 12, o.ev[12], qxz, 14, m12, 15);
+  M[13] = alone(13, o.ev[13]);
+  M[14] = alone(14, o.ev[14]);
+  M[15] = alone(15, o.ev[15]);
   const Split xr[1] = {rhos}, yr[1] = {C(18)};
   const I tl1 = dot_shift<64, 1>(xr, yr);
   const I tl6 = momentum(0), tl8 = momentum(1), tl10 = momentum(2);
@@ -737,6 +752,116 @@ __host__ __device__ __forceinline__ bool fx_core_int(const long long (&g)[NPOP],
     h[16] = bm - Q;
     h[17] = bm + Q;
   }
+  return true;
+}
+
+__host__ __device__ __forceinline__ bool fx_core_int(const long long (&g)[NPOP], long long fpx,
+                                                     long long fpy, long long fpz, long long Fx,
+                                                     long long Fy, long long Fz,
+                                                     const RatesT<double>& r,
+                                                     long long (&h)[NPOP], long long bias = 0) {
+  typedef long long I;
+  FxSums o;
+  fx_sums(g, o);
+  // macrovar: u = sum c f + F_prev / 2, exact at 2^-kFxIn
+  constexpr int sh = kFxF - kFxIn + 1;
+  auto half = [](long long v) { return (v + (1LL << (sh - 1))) >> sh; };
+  const I ux = o.jx + half(fpx);
+  const I uy = o.jy + half(fpy);
+  const I uz = o.jz + half(fpz);
+  {
+    // |u| < 2^-2 and |F| < 2^-9, on the high words (the bounds' low words are
+    // zero, as for the input test of collide_fx_fixed_int)
+    constexpr unsigned ulim = 1u << (kFxIn - 2 - 32);
+    constexpr unsigned flim = 1u << (kFxF - 9 - 32);
+    auto hw = [](long long v) { return (unsigned)((unsigned long long)v >> 32); };
+    const unsigned bad = ((hw(ux) + ulim) | (hw(uy) + ulim) | (hw(uz) + ulim)) & ~(2 * ulim - 1);
+    const unsigned badf = ((hw(Fx) + flim) | (hw(Fy) + flim) | (hw(Fz) + flim)) & ~(2 * flim - 1);
+    if (bad | badf) return false;
+  }
+  constexpr int su = kFxUU - kFxIn;
+  const Split U[3] = {split(ux << su), split(uy << su), split(uz << su)};
+  const Split F[3] = {split(Fx), split(Fy), split(Fz)};
+  return fx_relax(o, o.rho, U, U, F, F, r, h, bias);
+}
+
+// collision_MRT of FP64 populations with the density and velocity given (its
+// own subroutine takes them from macrovar's arrays), in the integer core at a
+// scale of the node's own: 2^j finer than fx_core_int's, with the largest j
+// for which populations, velocity, density and force stay in its ranges, so
+// that 54 bits and more below the node's largest population are kept (FP64
+// has 53 below each).  sum_rho: the density is the populations' sum (rho is
+// set to it).  False, with f as it was, when a value is not finite or too
+// large, or the node is so quiet that j would pass 40 (its populations below
+// 2^-44): the caller then takes the FP64 form.
+__host__ __device__ __forceinline__ bool collide_fx_at(double (&f)[NPOP], bool sum_rho, double& rho,
+                                                       double ux, double uy, double uz, double fx,
+                                                       double fy, double fz,
+                                                       const RatesT<double>& r) {
+  auto most = [](int a, int b) { return a > b ? a : b; };
+  int ef = 0;
+#pragma unroll
+  for (int q = 0; q < NPOP; ++q) ef = most(ef, fx_exponent(f[q]));
+  const int eu = most(fx_exponent(ux), most(fx_exponent(uy), fx_exponent(uz)));
+  const int eF = most(fx_exponent(fx), most(fx_exponent(fy), fx_exponent(fz)));
+  // |f| < 2^(-4 - j), |u| < 2^(-2 - j), |F| < 2^(-9 - j), |rho| < 2^(-1 - j)
+  // as fixed point: 2^54, 2^62, 2^61, 2^57
+  int j = 1018 - ef;
+  j = -most(-j, most(eu - 1020, eF - 1013));
+  if (!sum_rho) j = -most(-j, fx_exponent(rho) - 1021);
+  if (j < 0 || j > 40) return false;
+  long long g[NPOP], h[NPOP];
+#pragma unroll
+  for (int q = 0; q < NPOP; ++q) g[q] = fx_from_k(f[q], kFxIn + j);
+  FxSums o;
+  fx_sums(g, o);
+  const long long u[3] = {fx_from_k(ux, kFxUU + j), fx_from_k(uy, kFxUU + j), fx_from_k(uz, kFxUU + j)};
+  const long long w[3] = {fx_from_k(fx, kFxF), fx_from_k(fy, kFxF), fx_from_k(fz, kFxF)};
+  const long long half = (1LL << j) >> 1;
+  const Split U[3] = {split(u[0]), split(u[1]), split(u[2])};
+  const Split V[3] = {split((u[0] + half) >> j), split((u[1] + half) >> j), split((u[2] + half) >> j)};
+  const Split F[3] = {split(w[0]), split(w[1]), split(w[2])};
+  const Split Fj[3] = {split((long long)((unsigned long long)w[0] << j)),
+                       split((long long)((unsigned long long)w[1] << j)),
+                       split((long long)((unsigned long long)w[2] << j))};
+  const long long rho_i = sum_rho ? o.rho : fx_from_k(rho, kFxIn + j);
+  if (!fx_relax(o, rho_i, U, V, F, Fj, r, h, 0)) return false;
+  if (sum_rho) rho = fx_to_k(o.rho, kFxIn + j);
+#pragma unroll
+  for (int q = 0; q < NPOP; ++q) f[q] = fx_to_k(h[q], kFxOut + j);
+  return true;
+}
+
+// Density and momentum of FP64 populations as exact integer sums at a scale
+// of the node's own (the largest population at 2^58, so nothing below 2^-58 of
+// it is lost), rounded once: 4 conversions back instead of the ~40 FP64 adds
+// that bound macrovar on this GPU's FP64 pipe.  False for values that are not
+// finite or all below 2^-900.
+__host__ __device__ __forceinline__ bool fx_moments(const double (&f)[NPOP], double& rho, double& jx,
+                                                    double& jy, double& jz) {
+  int ef = 0;
+#pragma unroll
+  for (int q = 0; q < NPOP; ++q) {
+    const int e = fx_exponent(f[q]);
+    ef = ef > e ? ef : e;
+  }
+  if (ef >= 2047 || ef < 123) return false;
+  const int K = 1022 + 58 - ef;
+  long long g[NPOP];
+#pragma unroll
+  for (int q = 0; q < NPOP; ++q) g[q] = fx_from_k(f[q], K);
+  long long s = g[0], x = 0, y = 0, z = 0;
+#pragma unroll
+  for (int q = 1; q < NPOP; ++q) {
+    s += g[q];
+    x += cix(q) * g[q];
+    y += ciy(q) * g[q];
+    z += ciz(q) * g[q];
+  }
+  rho = fx_to_k(s, K);
+  jx = fx_to_k(x, K);
+  jy = fx_to_k(y, K);
+  jz = fx_to_k(z, K);
   return true;
 }
 

@@ -465,9 +465,13 @@ __global__ void k_stream(Geometry g, const T* __restrict__ fin, T* __restrict__ 
 }
 
 // collision_MRT alone (per-subroutine entry), in place, using the stored
-// macroscopic arrays as the reference does
-template <typename T>
-__global__ void k_collision(Geometry g, Rates r, T* __restrict__ f,
+// macroscopic arrays as the reference does.  FX (FP64): in the integer core at
+// the node's own scale (collide_fx_at), the literal FP64 form for the nodes it
+// declines.  The literal form's ~615 FP64 instructions a node took 1.75 ms at
+// 128^3, two thirds of a step of the subroutine loop there (150 spheres: 2.4
+// -> 0.69 ms a step with this and macrovar's integer sums).
+template <typename T, bool FX = false>
+__global__ void __launch_bounds__(128, FX ? 4 : 1) k_collision(Geometry g, Rates r, RatesT<double> rt, T* __restrict__ f,
                             const int32_t* __restrict__ isnodes, ForceView<T> fv,
                             const T* __restrict__ rho, const T* __restrict__ ux,
                             const T* __restrict__ uy, const T* __restrict__ uz) {
@@ -482,9 +486,105 @@ __global__ void k_collision(Geometry g, Rates r, T* __restrict__ f,
   for (int q = 0; q < NPOP; ++q) fl[q] = f[q * N + n];
   T fx, fy, fz;
   body_force(fv, g, x, y, z, fx, fy, fz);
-  collide_mrt(fl, rho[n], ux[n], uy[n], uz[n], fx, fy, fz, r);
+  bool done = false;
+  if constexpr (FX) {
+    double rho9 = rho[n];
+    done = collide_fx_at(fl, false, rho9, ux[n], uy[n], uz[n], fx, fy, fz, rt);
+  }
+  if (!done) {
+    if constexpr (FX) {
+      // read again rather than kept in registers through the integer core
+#pragma unroll
+      for (int q = 0; q < NPOP; ++q) fl[q] = f[q * N + n];
+    }
+    collide_mrt(fl, rho[n], ux[n], uy[n], uz[n], fx, fy, fz, r);
+  }
 #pragma unroll
   for (int q = 0; q < NPOP; ++q) f[q * N + n] = fl[q];
+}
+
+// One iteration of the pre-relaxation loop in one pass (FP64): rhoupdat of the
+// populations as they stand with the largest density change of the iteration
+// that made them, then the next iteration's collision_MRT (velocity held) and
+// streaming into the other buffer: 2 x 19 + 5 values a node instead of the
+// 2 x 42 + 20 of three kernels (128^3: 1.96 -> 0.27 ms).
+// first: the collision uses the stored density (no iteration made these
+// populations).  before: the change the previous pass found; when it is within
+// eps or not finite the loop has ended, and this pass does nothing.
+template <bool CHANNEL>
+__global__ void __launch_bounds__(128, 4) k_relax(Geometry g, Rates r, RatesT<double> rt, const double* __restrict__ fin,
+                            double* __restrict__ fout, const int32_t* __restrict__ isnodes,
+                            ForceView<double> fv, double* __restrict__ rho,
+                            const double* __restrict__ ux, const double* __restrict__ uy,
+                            const double* __restrict__ uz, bool first,
+                            const unsigned long long* __restrict__ before,
+                            unsigned long long* __restrict__ change, double eps) {
+  if (before) {
+    const double e = __longlong_as_double((long long)*before);
+    if (e <= eps || isinf(e)) return;
+  }
+  const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  const int y = blockIdx.y, z = blockIdx.z;
+  const int nx = g.nx, nxy = g.nx * g.ny, N = (int)g.N;
+  const int n = x + nx * y + nxy * z;
+  double d = 0.0;
+  if (x < nx) {
+    double f[NPOP];
+#pragma unroll
+    for (int q = 0; q < NPOP; ++q) f[q] = fin[(size_t)q * N + n];
+    const double old = rho[n];
+    double rho9 = old;
+    const bool solid = isnodes[n] >= 0;
+    bool done = false;
+    double fx = 0.0, fy = 0.0, fz = 0.0, u1 = 0.0, u2 = 0.0, u3 = 0.0;
+    if (!solid) {
+      body_force(fv, g, x, y, z, fx, fy, fz);
+      u1 = ux[n]; u2 = uy[n]; u3 = uz[n];
+      done = collide_fx_at(f, !first, rho9, u1, u2, u3, fx, fy, fz, rt);
+    }
+    if (!done) {
+      // read again rather than kept in registers through the integer core
+#pragma unroll
+      for (int q = 0; q < NPOP; ++q) f[q] = fin[(size_t)q * N + n];
+      if (!first) {
+        double jx, jy, jz;
+        if (!fx_moments(f, rho9, jx, jy, jz)) {
+          rho9 = f[0];
+#pragma unroll
+          for (int q = 1; q < NPOP; ++q) rho9 = rho9 + f[q];
+        }
+      }
+      if (!solid) collide_mrt(f, rho9, u1, u2, u3, fx, fy, fz, r);
+    }
+    if (!first) {
+      d = fabs(rho9 - old);
+      if (!(d == d)) d = __longlong_as_double(0x7ff0000000000000LL);  // NaN -> +inf
+      rho[n] = rho9;
+    }
+    const int oxp = (x == nx - 1) ? 1 - nx : 1, oxm = (x == 0) ? nx - 1 : -1;
+    const int oyp = (y == g.ny - 1) ? nx - nxy : nx, oym = (y == 0) ? nxy - nx : -nx;
+    const int ozp = (z == g.nz - 1) ? nxy - N : nxy, ozm = (z == 0) ? N - nxy : -nxy;
+#pragma unroll
+    for (int q = 0; q < NPOP; ++q) {
+      const int cx = cix(q), cy = ciy(q), cz = ciz(q);
+      if (CHANNEL && ((cx == -1 && x == 0) || (cx == 1 && x == nx - 1))) {
+        fout[(size_t)ipopp(q) * N + n] = f[q];
+        continue;
+      }
+      const int off = (cx > 0 ? oxp : (cx < 0 ? oxm : 0)) + (cy > 0 ? oyp : (cy < 0 ? oym : 0)) +
+                      (cz > 0 ? ozp : (cz < 0 ? ozm : 0));
+      fout[(size_t)q * N + (n + off)] = f[q];
+    }
+  }
+  if (first) return;
+  // the largest change as the bits of a non-negative double (ordered alike)
+  unsigned long long m = (unsigned long long)__double_as_longlong(d);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned long long t = __shfl_xor_sync(0xffffffffu, m, o);
+    m = t > m ? t : m;
+  }
+  if ((threadIdx.x & 31) == 0 && m) atomicMax(change, m);
 }
 
 // macrovar, B/collision.f90:232-332 (solid branch with nearest image; the
@@ -503,7 +603,9 @@ __global__ void k_macrovar(Geometry g, const T* __restrict__ f,
 #pragma unroll
   for (int q = 0; q < NPOP; ++q) fl[q] = f[q * N + n];
   T rho9, ux9, uy9, uz9, fx, fy, fz;
-  moments(fl, rho9, ux9, uy9, uz9);
+  bool done = false;
+  if constexpr (sizeof(T) == 8) done = fx_moments(fl, rho9, ux9, uy9, uz9);
+  if (!done) moments(fl, rho9, ux9, uy9, uz9);
   body_force(fv, g, x, y, z, fx, fy, fz);
   T u1 = ux9 + fx * T(0.5), u2 = uy9 + fy * T(0.5), u3 = uz9 + fz * T(0.5), rr = rho9;
   int id = isnodes[n];
@@ -566,6 +668,41 @@ __global__ void __launch_bounds__(256) k_rhoupdat_maxdiff(Geometry g, const T* _
     for (int w = 1; w < (int)(blockDim.x >> 5); ++w) m = fmax(m, wm[w]);
     atomicMax(maxbits, (unsigned long long)__double_as_longlong(m));
   }
+}
+
+// the last rhoupdat of the pre-relaxation's passes (k_relax without the next
+// collision)
+__global__ void __launch_bounds__(256) k_rhoupdat_change(Geometry g, const double* __restrict__ f,
+                                                         double* __restrict__ rho,
+                                                         const unsigned long long* __restrict__ before,
+                                                         unsigned long long* __restrict__ change,
+                                                         double eps) {
+  if (before) {
+    const double e = __longlong_as_double((long long)*before);
+    if (e <= eps || isinf(e)) return;
+  }
+  const long long n = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  double d = 0.0;
+  if (n < g.N) {
+    double fl[NPOP], rho9, jx, jy, jz;
+#pragma unroll
+    for (int q = 0; q < NPOP; ++q) fl[q] = f[q * g.N + n];
+    if (!fx_moments(fl, rho9, jx, jy, jz)) {
+      rho9 = fl[0];
+#pragma unroll
+      for (int q = 1; q < NPOP; ++q) rho9 = rho9 + fl[q];
+    }
+    d = fabs(rho9 - rho[n]);
+    if (!(d == d)) d = __longlong_as_double(0x7ff0000000000000LL);  // NaN -> +inf
+    rho[n] = rho9;
+  }
+  unsigned long long m = (unsigned long long)__double_as_longlong(d);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned long long t = __shfl_xor_sync(0xffffffffu, m, o);
+    m = t > m ? t : m;
+  }
+  if ((threadIdx.x & 31) == 0 && m) atomicMax(change, m);
 }
 
 // initpop, B/initial.f90:14-26 (rho' = 0)
@@ -885,8 +1022,39 @@ void launch_macrovar(const Geometry& g, const T* f, const int32_t* isnodes,
 template <typename T>
 void launch_collision(const Geometry& g, const Rates& r, T* f, const int32_t* isnodes,
                       const ForceView<T>& fv, const T* rho, const T* ux, const T* uy,
-                      const T* uz, cudaStream_t s) {
-  { k_collision<T><<<row_grid(g, 128), 128, 0, s>>>(g, r, f, isnodes, fv, rho, ux, uy, uz); count_launch(); }
+                      const T* uz, bool fx, cudaStream_t s) {
+  const RatesT<double> rt = rates_t<double>(r);
+  if constexpr (sizeof(T) == 8) {
+    if (fx && rt.int_ok) {
+      k_collision<T, true><<<row_grid(g, 128), 128, 0, s>>>(g, r, rt, f, isnodes, fv, rho, ux, uy, uz);
+      count_launch();
+      return;
+    }
+  }
+  { k_collision<T><<<row_grid(g, 128), 128, 0, s>>>(g, r, rt, f, isnodes, fv, rho, ux, uy, uz); count_launch(); }
+}
+
+bool launch_relax(const Geometry& g, const Rates& r, const double* fin, double* fout,
+                  const int32_t* isnodes, const ForceView<double>& fv, double* rho,
+                  const double* ux, const double* uy, const double* uz, bool first,
+                  const unsigned long long* before, unsigned long long* change, double eps,
+                  cudaStream_t s) {
+  const RatesT<double> rt = rates_t<double>(r);
+  if (!rt.int_ok) return false;
+  auto launch = [&](auto kern) {
+    kern<<<row_grid(g, 128), 128, 0, s>>>(g, r, rt, fin, fout, isnodes, fv, rho, ux, uy, uz, first,
+                                          before, change, eps);
+  };
+  g.channel ? launch(k_relax<true>) : launch(k_relax<false>);
+  count_launch();
+  return true;
+}
+
+void launch_rhoupdat_change(const Geometry& g, const double* f, double* rho,
+                            const unsigned long long* before, unsigned long long* change,
+                            double eps, cudaStream_t s) {
+  k_rhoupdat_change<<<blocks_for(g.N, 256), 256, 0, s>>>(g, f, rho, before, change, eps);
+  count_launch();
 }
 
 template <typename T>
@@ -1013,7 +1181,7 @@ void launch_forcing_tables(const Geometry& g, const ForcingDev* st, const T* ytw
                                    cudaStream_t);                                           \
   template void launch_collision<T>(const Geometry&, const Rates&, T*, const int32_t*,      \
                                     const ForceView<T>&, const T*, const T*, const T*,      \
-                                    const T*, cudaStream_t);                                \
+                                    const T*, bool, cudaStream_t);                          \
   template void launch_streaming<T>(const Geometry&, const T*, T*, cudaStream_t);           \
   template void launch_rhoupdat<T>(const Geometry&, const T*, T*, cudaStream_t);            \
   template void launch_rhoupdat_maxdiff<T>(const Geometry&, const T*, T*, unsigned long long*, \

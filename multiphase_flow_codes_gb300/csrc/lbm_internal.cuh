@@ -212,7 +212,17 @@ void launch_macrovar(const Geometry& g, const T* f, const int32_t* isnodes,
 template <typename T>
 void launch_collision(const Geometry& g, const Rates& r, T* f, const int32_t* isnodes,
                       const ForceView<T>& fv, const T* rho, const T* ux, const T* uy,
-                      const T* uz, cudaStream_t s);
+                      const T* uz, bool fx, cudaStream_t s);
+// one pass of the pre-relaxation loop (k_relax); false: these rates take the
+// three kernels
+bool launch_relax(const Geometry& g, const Rates& r, const double* fin, double* fout,
+                  const int32_t* isnodes, const ForceView<double>& fv, double* rho,
+                  const double* ux, const double* uy, const double* uz, bool first,
+                  const unsigned long long* before, unsigned long long* change, double eps,
+                  cudaStream_t s);
+void launch_rhoupdat_change(const Geometry& g, const double* f, double* rho,
+                            const unsigned long long* before, unsigned long long* change,
+                            double eps, cudaStream_t s);
 template <typename T>
 void launch_streaming(const Geometry& g, const T* fin, T* fout, cudaStream_t s);
 template <typename T>
