@@ -533,10 +533,8 @@ void particle_phase(lbm_ctx* c, T* f_plain) {
   }
   prof_begin(c);
   if (!pre) launch_lubforce(c->g, c->npart, c->pp, mstate(c), c->stream);
-  const ParticleView pv = pview(c);
-  const bool ovl_aux = launch_move_redistribute(c->g, c->npart, c->pp, mstate(c), c->status,
-                                                c->stream, c->aux, c->ev_aux_fork, c->ev_aux_join,
-                                                &pv, &c->links);
+  const bool ovl_aux = launch_move_redistribute(c->g, c->npart, c->pp, mstate(c), c->links, c->status,
+                                                c->stream, c->aux, c->ev_aux_fork, c->ev_aux_join);
   prof_end(c, LBM_PHASE_PARTICLES);
   int nf = 1 - c->fcur;
   prof_begin(c);

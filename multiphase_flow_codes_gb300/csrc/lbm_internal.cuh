@@ -368,17 +368,16 @@ void launch_move(const Geometry& g, int npart, const PartParams& pp, MoveState m
                  cudaStream_t s);
 void launch_redistribute(const Geometry& g, int npart, const PartParams& pp, MoveState ms,
                          DevStatus* st, cudaStream_t s);
-// launch_move then launch_redistribute in two launches: the move and the wrap
-// of a particle in one thread, then the overlap check (which also ends the
-// first move).  The check only reports; with an aux stream it runs there,
+// launch_move, launch_redistribute and beads_links' nearest-image sweeps
+// (launch_links then skips them) in two launches: the move, the wrap and the
+// sweep of a coordinate in one thread, then the overlap check (which also ends
+// the first move).  The check only reports; with an aux stream it runs there,
 // forked after the move by `fork` and recorded into `join`, beside the link
 // kernels that follow on s (returns true: the caller joins `join`).
-// With pv and ls, the same launch also runs beads_links' nearest-image
-// sweeps of every moved particle (launch_links then skips them).
 bool launch_move_redistribute(const Geometry& g, int npart, const PartParams& pp, MoveState ms,
-                              DevStatus* st, cudaStream_t s, cudaStream_t aux = nullptr,
-                              cudaEvent_t fork = nullptr, cudaEvent_t join = nullptr,
-                              const ParticleView* pv = nullptr, LinkSlab* ls = nullptr);
+                              const LinkSlab& ls, DevStatus* st, cudaStream_t s,
+                              cudaStream_t aux = nullptr, cudaEvent_t fork = nullptr,
+                              cudaEvent_t join = nullptr);
 // refill events of one step: node index and particle id per event
 struct FillList {
   int32_t* node;

@@ -21,6 +21,7 @@
 
 #include "lbm_internal.cuh"
 #include "lbm_collide.cuh"  // the fixed-point population format
+#include "lbm_sweeps.cuh"
 
 namespace lbm {
 
@@ -54,87 +55,6 @@ __device__ __forceinline__ R near_img_t(R c, R p, int n, int nh) {
   if ((c - p) > R(nh)) c = c - R(n);
   if ((c - p) < -R(nh)) c = c + R(n);
   return c;
-}
-
-// The reference's beads_links keeps shifting the particle centre toward the
-// current point and never resets it inside its loop nest
-// (B/partlib.f90:961-982): at point p_j = j - 0.5 of a sweep j = 1..n it
-// applies "if (c - p > n/2) c -= n; if (c - p < -n/2) c += n" to the value
-// left by the previous point.  fl(c - p) is monotone in p, so both shift
-// predicates are monotone along a sweep and the points where a shift fires
-// are found by bisection instead of visiting every point.
-// The points of one sweep where the shifted coordinate changes, with the
-// value after each change: a sweep starting from c changes at most a few
-// times (a shift down at the first point, a shift up once c - p drops
-// below -n/2), so any point's value is a lookup in this short list.
-constexpr int MAXEV = 6;
-struct SweepEv {
-  int nev;
-  int ok;
-  int j[MAXEV];
-  double v[MAXEV];
-  double v0;
-};
-static_assert(7 * sizeof(SweepEv) <= kSweepBytes, "sweep slab too small");
-__device__ SweepEv sweep_events(double c, int n, int nh) {
-  SweepEv s;
-  s.nev = 0;
-  s.ok = 1;
-  s.v0 = c;
-  const double dn = (double)n, dnh = (double)nh;
-  int j = 1;
-  for (int guard = 0; guard < 16; ++guard) {
-    const double p = (double)j - 0.5;
-    const double before = c;
-    if ((c - p) > dnh) c = c - dn;
-    if ((c - p) < -dnh) c = c + dn;
-    if (__double_as_longlong(c) != __double_as_longlong(before)) {
-      if (s.nev < MAXEV) { s.j[s.nev] = j; s.v[s.nev] = c; ++s.nev; } else s.ok = 0;
-    }
-    if (j >= n) return s;
-    int jn = n + 1;
-    const double p1 = (double)(j + 1) - 0.5;
-    if ((c - p1) > dnh) {
-      jn = j + 1;
-    } else if ((c - ((double)n - 0.5)) < -dnh) {
-      // the first point m in [j + 1, n] where the shift up fires.  In exact
-      // arithmetic that is the first m > c + n/2 + 1/2, and fl(c - p) is
-      // within an ulp of c - p, so the FP64 first point lies within two of
-      // floor(c + n/2 + 1/2) + 1: scan from two below it with the
-      // reference's expression (monotone in m) after checking that the start
-      // is not past it; bisect where either check fails (not expected).
-      auto up = [&](int m) { return (c - ((double)m - 0.5)) < -dnh; };
-      int lo = j + 1, hi = n;
-      int m = (int)floor(c + dnh + 0.5) - 1;
-      m = m < lo ? lo : (m > hi ? hi : m);
-      bool found = false;
-      if (m == lo || !up(m - 1)) {
-        for (int t = 0; t < 6 && m <= hi; ++t, ++m)
-          if (up(m)) { found = true; break; }
-        if (!found) lo = m;
-      } else {
-        hi = m - 1;
-      }
-      if (!found) {
-        while (lo < hi) {
-          int mid = (lo + hi) >> 1;
-          if (up(mid)) hi = mid; else lo = mid + 1;
-        }
-        m = lo;
-      }
-      jn = m;
-    }
-    if (jn > n) return s;
-    j = jn;
-  }
-  s.ok = 0;
-  return s;
-}
-__device__ __forceinline__ double sweep_value(const SweepEv& s, int jq) {
-  double v = s.v0;
-  for (int e = 0; e < s.nev; ++e)
-    if (s.j[e] <= jq) v = s.v[e];
-  return v;
 }
 
 // candidate indices (1-based) along one axis: the union, in ascending order,
@@ -205,48 +125,59 @@ constexpr float kDecide = 4e-3f;
 // from the second sweep on unless the centre lies within an ulp of
 // n/2 - 1/2, which sweep_ok reports.  FP64 and serial by nature; run for all
 // particles at once rather than inside each link block.
-__device__ __forceinline__ void k_link_sweeps_body(int bx, int gx, Geometry g, ParticleView pv, LinkSlab ls) {
-  const int t = bx * blockDim.x + threadIdx.x;
-  if (t >= 3 * pv.npart) return;
-  const int p = t / 3, axis = t - 3 * p;
+// the coordinate that sweep `axis` (0: y, 1: x, 2: z) follows
+__device__ __forceinline__ int sweep_coord(int axis) { return axis == 0 ? 1 : (axis == 1 ? 0 : 2); }
+__device__ __forceinline__ void link_sweeps(int p, int axis, double c0, const Geometry& g, LinkSlab ls) {
   SweepEv* out = reinterpret_cast<SweepEv*>(static_cast<char*>(ls.sweeps) + (size_t)p * kSweepBytes);
-  const double c0 = pv.ypglb[3 * p + (axis == 0 ? 1 : axis == 1 ? 0 : 2)];
   int ok = 1;
   if (!isfinite(c0)) {
     ok = 0;
   } else {
     // The three axes in one instruction stream: y and x take three start
-    // states and the fixed-point check (four sweeps), z one sweep; the z
-    // lanes run the y and x lanes' four rounds with them and keep only the
-    // first, so that a warp pays for four serial sweeps rather than five
-    // (FP64 issues at 2 lanes per clock per SM whatever the active lanes).
+    // states and the fixed-point check (four sweeps), z one sweep.
     const bool xwall = axis == 1 && g.channel;  // no x sweep in the channel
     const int n = axis == 0 ? g.ny : (axis == 1 ? g.nx : g.nz);
     const int nh = axis == 0 ? g.nyh : (axis == 1 ? g.nxh : g.nzh);
     SweepEv* o = out + 3 * axis;
     double c = c0;
-    for (int s = 0; s < 4; ++s) {
-      const SweepEv e = sweep_events(c, n, nh);
-      const double next = sweep_value(e, n);
-      if (!xwall) {
-        if (axis == 2) {
-          if (s == 0) { o[0] = e; ok = e.ok; }
-        } else if (s < 3) {
-          o[s] = e;
-          ok &= e.ok;
-        } else if (next != c) {
-          ok = 0;
-        }
+    const int keep = xwall ? 0 : (axis == 2 ? 1 : 3);
+    for (int s = 0; s < 4 && s <= keep && keep > 0; ++s) {
+      if (s == keep && axis == 2) break;
+      const double start = c;
+      SweepEv e;
+      if (!sweep_fast(c, n, nh, &e)) {
+        e = sweep_events(c, n, nh);
+        c = sweep_value(e, n);
       }
-      c = next;
+      if (s < keep) {
+        o[s].nev = e.nev;
+        o[s].ok = e.ok;
+        o[s].v0 = e.v0;
+        for (int k = 0; k < e.nev; ++k) {
+          o[s].j[k] = e.j[k];
+          o[s].v[k] = e.v[k];
+        }
+        ok &= e.ok;
+      } else if (c != start) {
+        ok = 0;
+      }
     }
     if (xwall) {
-      SweepEv e;
-      e.nev = 0; e.ok = 1; e.v0 = c0;
-      out[3] = e; out[4] = e; out[5] = e;
+#pragma unroll
+      for (int s = 3; s < 6; ++s) {
+        out[s].nev = 0;
+        out[s].ok = 1;
+        out[s].v0 = c0;
+      }
     }
   }
   ls.sweep_ok[3 * p + axis] = ok;
+}
+__device__ __forceinline__ void k_link_sweeps_body(int bx, int gx, Geometry g, ParticleView pv, LinkSlab ls) {
+  const int t = bx * blockDim.x + threadIdx.x;
+  if (t >= 3 * pv.npart) return;
+  const int p = t / 3, axis = t - 3 * p;
+  link_sweeps(p, axis, pv.ypglb[3 * p + sweep_coord(axis)], g, ls);
 }
 __global__ void k_link_sweeps(Geometry g, ParticleView pv, LinkSlab ls) {
   k_link_sweeps_body(blockIdx.x, gridDim.x, g, pv, ls);
@@ -326,8 +257,10 @@ __device__ __forceinline__ void k_links_body(int bx, int gx, Geometry g, Particl
   // planes at Y2) and of the x sweep (rows likewise: x0, X1, X2), and for the
   // single z sweep.
   __shared__ SweepEv sev[7];  // 0..2: y states, 3..5: x states, 6: z
-  if (tid < 7) sev[tid] = reinterpret_cast<const SweepEv*>(
-      static_cast<const char*>(ls.sweeps) + (size_t)p * kSweepBytes)[tid];
+  static_assert(sizeof(sev) % 4 == 0 && sizeof(sev) <= PB * 4, "one word a thread");
+  if (tid < (int)(sizeof(sev) / 4))
+    reinterpret_cast<int*>(sev)[tid] = reinterpret_cast<const int*>(
+        static_cast<const char*>(ls.sweeps) + (size_t)p * kSweepBytes)[tid];
   if (tid == 0) {
     const int32_t* ok = ls.sweep_ok + 3 * p;
     if (!(ok[0] && ok[1] && ok[2])) fixed_ok = 0;
@@ -1131,104 +1064,83 @@ __global__ void k_lubforce(Geometry g, int npart, PartParams pp, MoveState ms) {
   k_lubforce_body(blockIdx.x, gridDim.x, g, npart, pp, ms);
 }
 
-// beads_move, B/partlib.f90:2305-2370, one thread per particle.  Also saves
-// the pre-move centre (ypglbp, used by beads_filling).
-__device__ __forceinline__ void move_particle(int p, int npart, PartParams pp, MoveState ms) {
-  if (p >= npart) return;
+// beads_move, B/partlib.f90:2305-2370, one thread per particle and component
+// (the components do not mix): a third of the serial FP64 chain of a thread
+// per particle.  Also saves the pre-move centre (ypglbp, used by
+// beads_filling).  Returns the moved coordinate.
+__device__ __forceinline__ double move_component(int p, int c, const PartParams& pp, const MoveState& ms) {
   const bool first = *ms.first_move != 0;
   const double dt = 1.0;
-  double fp[3], fpp[3], dwdtn[3], domgdtn[3];
-  if (first) for (int c = 0; c < 3; ++c) ms.thetap[3 * p + c] = 0.0;
-  for (int c = 0; c < 3; ++c) {
-    ms.wpp[3 * p + c] = ms.wp[3 * p + c];
-    ms.omgpp[3 * p + c] = ms.omgp[3 * p + c];
-    ms.ypglbp[3 * p + c] = ms.ypglb[3 * p + c];
-  }
-  for (int c = 0; c < 3; ++c) fp[c] = ms.fHIp[3 * p + c] + ms.flubp[3 * p + c];
-  fp[1] = fp[1] + pp.body_force_y;
-  for (int c = 0; c < 3; ++c) fpp[c] = first ? fp[c] : ms.forcepp[3 * p + c];
-  for (int c = 0; c < 3; ++c) dwdtn[c] = 0.5 * (fp[c] + fpp[c]) / pp.amp;
-  for (int c = 0; c < 3; ++c) {
-    double dw = first ? dwdtn[c] : ms.dwdt[3 * p + c];
-    double wpp = ms.wpp[3 * p + c];
-    double w = wpp + 0.5 * dt * (dw + dwdtn[c]);
-    ms.wp[3 * p + c] = w;
-    ms.ypglb[3 * p + c] = ms.ypglb[3 * p + c] + 0.5 * dt * (w + wpp);
-  }
-  for (int c = 0; c < 3; ++c) {
-    double tq = ms.torqp[3 * p + c];
-    double tpp = first ? tq : ms.torqpp[3 * p + c];
-    domgdtn[c] = 0.5 * (tq + tpp) / pp.aip;
-  }
-  for (int c = 0; c < 3; ++c) {
-    double dom = first ? domgdtn[c] : ms.domgdt[3 * p + c];
-    double opp_ = ms.omgpp[3 * p + c];
-    double o = opp_ + 0.5 * dt * (dom + domgdtn[c]);
-    ms.omgp[3 * p + c] = o;
-    ms.thetap[3 * p + c] = ms.thetap[3 * p + c] + 0.5 * dt * (o + opp_);
-  }
-  for (int c = 0; c < 3; ++c) {
-    ms.dwdt[3 * p + c] = dwdtn[c];
-    ms.domgdt[3 * p + c] = domgdtn[c];
-    ms.forcep[3 * p + c] = fp[c];
-    ms.forcepp[3 * p + c] = fp[c];
-    ms.torqpp[3 * p + c] = ms.torqp[3 * p + c];
-  }
+  const int i = 3 * p + c;
+  const double y0 = ms.ypglb[i], wpp = ms.wp[i], opp = ms.omgp[i], tq = ms.torqp[i];
+  double fp = ms.fHIp[i] + ms.flubp[i];
+  if (c == 1) fp = fp + pp.body_force_y;
+  const double fpp = first ? fp : ms.forcepp[i];
+  const double dwdtn = 0.5 * (fp + fpp) / pp.amp;
+  const double dw = first ? dwdtn : ms.dwdt[i];
+  const double w = wpp + 0.5 * dt * (dw + dwdtn);
+  const double y = y0 + 0.5 * dt * (w + wpp);
+  const double tpp = first ? tq : ms.torqpp[i];
+  const double domgdtn = 0.5 * (tq + tpp) / pp.aip;
+  const double dom = first ? domgdtn : ms.domgdt[i];
+  const double o = opp + 0.5 * dt * (dom + domgdtn);
+  const double th = first ? 0.0 : ms.thetap[i];
+  ms.wpp[i] = wpp;
+  ms.omgpp[i] = opp;
+  ms.ypglbp[i] = y0;
+  ms.wp[i] = w;
+  ms.ypglb[i] = y;
+  ms.omgp[i] = o;
+  ms.thetap[i] = th + 0.5 * dt * (o + opp);
+  ms.dwdt[i] = dwdtn;
+  ms.domgdt[i] = domgdtn;
+  ms.forcep[i] = fp;
+  ms.forcepp[i] = fp;
+  ms.torqpp[i] = tq;
+  return y;
 }
-__device__ __forceinline__ void k_move_body(int bx, int gx, int npart, PartParams pp, MoveState ms) {
-  move_particle(bx * blockDim.x + threadIdx.x, npart, pp, ms);
+__device__ __forceinline__ void k_move_body(int bx, int npart, const PartParams& pp, const MoveState& ms) {
+  const int t = bx * blockDim.x + threadIdx.x;
+  if (t < 3 * npart) move_component(t / 3, t % 3, pp, ms);
 }
 __global__ void k_move(int npart, PartParams pp, MoveState ms) {
-  k_move_body(blockIdx.x, gridDim.x, npart, pp, ms);
+  k_move_body(blockIdx.x, npart, pp, ms);
 }
 
 __global__ void k_clear_first(int* first_move) { *first_move = 0; }
 
-// beads_redistribute's periodic wrap, B/partlib.f90:2600-2613
-__device__ __forceinline__ void wrap_particle(int p, Geometry g, int npart, MoveState ms) {
-  if (p >= npart) return;
-  double* y = ms.ypglb + 3 * p;
-  double xc = y[0], yc = y[1], zc = y[2];
-  if (!g.channel) {
-    if (xc >= (double)g.nx) y[0] = y[0] - (double)g.nx;
-    if (xc < 0.0) y[0] = y[0] + (double)g.nx;
-  }
-  if (yc >= (double)g.ny) y[1] = y[1] - (double)g.ny;
-  if (yc < 0.0) y[1] = y[1] + (double)g.ny;
-  if (zc >= (double)g.nz) y[2] = y[2] - (double)g.nz;
-  if (zc < 0.0) y[2] = y[2] + (double)g.nz;
-}
-__device__ __forceinline__ void k_wrap_body(int bx, int gx, Geometry g, int npart, MoveState ms) {
-  wrap_particle(bx * blockDim.x + threadIdx.x, g, npart, ms);
+// beads_redistribute's periodic wrap of one coordinate, B/partlib.f90:2600-2613
+__device__ __forceinline__ double wrap_coord(double v, int c, const Geometry& g) {
+  if (c == 0 && g.channel) return v;
+  const int n = c == 0 ? g.nx : (c == 1 ? g.ny : g.nz);
+  double w = v;
+  if (v >= (double)n) w = w - (double)n;
+  if (v < 0.0) w = w + (double)n;
+  return w;
 }
 __global__ void k_wrap(Geometry g, int npart, MoveState ms) {
-  k_wrap_body(blockIdx.x, gridDim.x, g, npart, ms);
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < 3 * npart) ms.ypglb[t] = wrap_coord(ms.ypglb[t], t % 3, g);
 }
-// beads_move, the wrap and the nearest-image sweeps of beads_links for
-// kMoveSweepParts particles per block of 3 kMoveSweepParts threads: thread
-// t < kMoveSweepParts moves and wraps particle kMoveSweepParts bx + t, then
-// thread t sweeps axis t % 3 of particle kMoveSweepParts bx + t / 3 (the
-// fused time step; the sweeps need only their own particle's new centre).
-// Eight particles (one warp) per block spread the serial FP64 chains over as
-// many SMs as there are blocks.
-constexpr int kMoveSweepParts = 8;
-constexpr int kMoveSweepThreads = 3 * kMoveSweepParts;
-__global__ void __launch_bounds__(kMoveSweepThreads) k_move_wrap_sweeps(Geometry g, int npart, PartParams pp,
-                                                                     MoveState ms, ParticleView pv,
-                                                                     LinkSlab ls) {
-  if (threadIdx.x < kMoveSweepParts) {
-    const int p = blockIdx.x * kMoveSweepParts + threadIdx.x;
-    move_particle(p, npart, pp, ms);
-    wrap_particle(p, g, npart, ms);
-  }
-  __syncthreads();
-  k_link_sweeps_body(blockIdx.x, gridDim.x, g, pv, ls);
+// beads_move, the wrap and the nearest-image sweeps of beads_links in one
+// launch, one thread per particle and axis: a sweep needs only its own
+// coordinate.  kSmallBlock threads a block spread the serial FP64 chains over
+// as many SMs as there are blocks.  Per step with its launch: 32 -> 18 us for
+// 1000 spheres (256^3, FP64), 26 -> 11 us for 16 (64^3).
+__device__ __forceinline__ void k_move_wrap_sweeps_body(int bx, const Geometry& g, int npart,
+                                                        const PartParams& pp, const MoveState& ms,
+                                                        const LinkSlab& ls) {
+  const int t = bx * blockDim.x + threadIdx.x;
+  if (t >= 3 * npart) return;
+  const int p = t / 3, axis = t - 3 * p, c = sweep_coord(axis);
+  const double y = move_component(p, c, pp, ms);
+  const double v = wrap_coord(y, c, g);
+  ms.ypglb[3 * p + c] = v;
+  link_sweeps(p, axis, v, g, ls);
 }
-// beads_move followed by beads_redistribute's wrap, each particle's thread
-// wrapping the centre it has just moved
-__global__ void k_move_wrap(Geometry g, int npart, PartParams pp, MoveState ms) {
-  k_move_body(blockIdx.x, gridDim.x, npart, pp, ms);
-  k_wrap_body(blockIdx.x, gridDim.x, g, npart, ms);
+__global__ void __launch_bounds__(kSmallBlock) k_move_wrap_sweeps(Geometry g, int npart, PartParams pp,
+                                                                MoveState ms, LinkSlab ls) {
+  k_move_wrap_sweeps_body(blockIdx.x, g, npart, pp, ms, ls);
 }
 
 // ovlpchk after a move (hgap = dist - 2 rad < 0 aborts the reference,
@@ -1596,25 +1508,22 @@ void launch_lubforce(const Geometry& g, int npart, const PartParams& pp, MoveSta
 void launch_move(const Geometry& g, int npart, const PartParams& pp, MoveState ms,
                  cudaStream_t s) {
   if (npart <= 0) return;
-  { k_move<<<(npart + kSmallBlock - 1) / kSmallBlock, kSmallBlock, 0, s>>>(npart, pp, ms); count_launch(); }
+  { k_move<<<(3 * npart + kSmallBlock - 1) / kSmallBlock, kSmallBlock, 0, s>>>(npart, pp, ms); count_launch(); }
   { k_clear_first<<<1, 1, 0, s>>>(ms.first_move); count_launch(); }
 }
 
 void launch_redistribute(const Geometry& g, int npart, const PartParams& pp, MoveState ms,
                          DevStatus* st, cudaStream_t s) {
   if (npart <= 0) return;
-  { k_wrap<<<(npart + kSmallBlock - 1) / kSmallBlock, kSmallBlock, 0, s>>>(g, npart, ms); count_launch(); }
+  { k_wrap<<<(3 * npart + kSmallBlock - 1) / kSmallBlock, kSmallBlock, 0, s>>>(g, npart, ms); count_launch(); }
   { k_overlap<<<(npart * 32 + 127) / 128, 128, 0, s>>>(g, npart, pp, ms, st, nullptr); count_launch(); }
 }
 
 bool launch_move_redistribute(const Geometry& g, int npart, const PartParams& pp, MoveState ms,
-                              DevStatus* st, cudaStream_t s, cudaStream_t aux, cudaEvent_t fork,
-                              cudaEvent_t join, const ParticleView* pv, LinkSlab* ls) {
+                              const LinkSlab& ls, DevStatus* st, cudaStream_t s, cudaStream_t aux,
+                              cudaEvent_t fork, cudaEvent_t join) {
   if (npart <= 0) return false;
-  if (pv && ls)
-    { k_move_wrap_sweeps<<<(npart + kMoveSweepParts - 1) / kMoveSweepParts, kMoveSweepThreads, 0, s>>>(g, npart, pp, ms, *pv, *ls); count_launch(); }
-  else
-    { k_move_wrap<<<(npart + kSmallBlock - 1) / kSmallBlock, kSmallBlock, 0, s>>>(g, npart, pp, ms); count_launch(); }
+  { k_move_wrap_sweeps<<<(3 * npart + kSmallBlock - 1) / kSmallBlock, kSmallBlock, 0, s>>>(g, npart, pp, ms, ls); count_launch(); }
   cudaStream_t so = s;
   if (aux) {
     cudaEventRecord(fork, s);
@@ -1661,10 +1570,9 @@ __global__ void k_lubforce_multi(const BoxParticles* boxes) {
   BOX_OR_RETURN((B.pv.npart * 32 + 127) / 128)
   k_lubforce_body(blockIdx.x, nblk, B.g, B.pv.npart, B.pp, B.ms);
 }
-__global__ void k_move_wrap_multi(const BoxParticles* boxes) {
-  BOX_OR_RETURN((B.pv.npart + kSmallBlock - 1) / kSmallBlock)
-  k_move_body(blockIdx.x, nblk, B.pv.npart, B.pp, B.ms);
-  k_wrap_body(blockIdx.x, nblk, B.g, B.pv.npart, B.ms);
+__global__ void __launch_bounds__(kSmallBlock) k_move_wrap_sweeps_multi(const BoxParticles* boxes) {
+  BOX_OR_RETURN((3 * B.pv.npart + kSmallBlock - 1) / kSmallBlock)
+  k_move_wrap_sweeps_body(blockIdx.x, B.g, B.pv.npart, B.pp, B.ms, B.ls);
 }
 __global__ void k_overlap_multi(const BoxParticles* boxes) {
   BOX_OR_RETURN((B.pv.npart * 32 + 127) / 128)
@@ -1685,10 +1593,6 @@ __global__ void k_reset_multi(const BoxParticles* boxes) {
     else mask[t - N] = 0u;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) *B.fl.count = 0;
-}
-__global__ void k_link_sweeps_multi(const BoxParticles* boxes) {
-  BOX_OR_RETURN((3 * B.pv.npart + kSmallBlock - 1) / kSmallBlock)
-  k_link_sweeps_body(blockIdx.x, nblk, B.g, B.pv, B.ls);
 }
 __global__ void __launch_bounds__(PB) k_links_multi(const BoxParticles* boxes) {
   BOX_OR_RETURN(B.pv.npart)
@@ -1716,11 +1620,10 @@ void launch_particle_step_multi(const BoxParticles* boxes, int nb, int max_npart
   k_bounce_multi<<<grid(max_npart), bounce_threads<float>(), 0, s>>>(boxes); count_launch();
   k_bounce_store_multi<<<grid(max_npart), PB, 0, s>>>(boxes); count_launch();
   k_lubforce_multi<<<grid((max_npart * 32 + 127) / 128), 128, 0, s>>>(boxes); count_launch();
-  k_move_wrap_multi<<<grid((max_npart + kSmallBlock - 1) / kSmallBlock), kSmallBlock, 0, s>>>(boxes); count_launch();
+  k_move_wrap_sweeps_multi<<<grid((3 * max_npart + kSmallBlock - 1) / kSmallBlock), kSmallBlock, 0, s>>>(boxes); count_launch();
   k_overlap_multi<<<grid((max_npart * 32 + 127) / 128), 128, 0, s>>>(boxes); count_launch();
   const long long rb = (max_reset + 256 * 8 - 1) / (256 * 8);
   k_reset_multi<<<grid(rb < 1024 ? rb : 1024), 256, 0, s>>>(boxes); count_launch();
-  k_link_sweeps_multi<<<grid((3 * max_npart + kSmallBlock - 1) / kSmallBlock), kSmallBlock, 0, s>>>(boxes); count_launch();
   k_links_multi<<<grid(max_npart), PB, 0, s>>>(boxes); count_launch();
   k_fill_detect_multi<<<grid(max_npart), PB, 0, s>>>(boxes); count_launch();
   k_fill_events_multi<<<grid(kFillBlocks), 128, 0, s>>>(boxes); count_launch();
