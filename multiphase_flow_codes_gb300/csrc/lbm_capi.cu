@@ -49,6 +49,9 @@ struct lbm_ctx {
   // bounce-back (particle_phase)
   cudaStream_t aux = nullptr;
   cudaEvent_t ev_aux_fork = nullptr, ev_aux_join = nullptr, ev_store = nullptr;
+  // the link lists of a fused step run on aux until ev_links (join_links)
+  cudaEvent_t ev_links = nullptr;
+  bool links_pending = false;
   bool aux_pending = false;
   bool store_pending = false;  // the bounce-back stores run on aux until ev_store
   bool prefetched = false;
@@ -495,9 +498,18 @@ void cancel_prefetch(lbm_ctx* c) {
   c->prefetched = false;
 }
 
+// The link lists of the last fused step, which nothing before the next
+// bounce-back reads, are complete on the main stream from here on.
+void join_links(lbm_ctx* c) {
+  if (!c->links_pending) return;
+  cudaStreamWaitEvent(c->stream, c->ev_links, 0);
+  c->links_pending = false;
+}
+
 // The part of the particle step that reads no post-collision populations:
 // the reset of the flag buffer beads_links fills next (last read by the
-// previous step's beads_filling) and beads_lubforce (positions only).  A
+// previous step's beads_filling) and of the refill list, and beads_lubforce
+// (positions only).  A
 // fused step launches it on the aux stream right after stream + collide, so
 // it runs beside the bounce-back; particle_phase joins it.
 void particle_prelude(lbm_ctx* c) {
@@ -505,6 +517,7 @@ void particle_prelude(lbm_ctx* c) {
   cudaEventRecord(c->ev_aux_fork, c->stream);
   cudaStreamWaitEvent(c->aux, c->ev_aux_fork, 0);
   reset_flags_on(c, 1 - c->fcur, c->aux);
+  cudaMemsetAsync(c->fill.count, 0, sizeof(int32_t), c->aux);
   launch_lubforce(c->g, c->npart, c->pp, mstate(c), c->aux);
   cudaEventRecord(c->ev_aux_join, c->aux);
   c->aux_pending = true;
@@ -538,14 +551,25 @@ void particle_phase(lbm_ctx* c, T* f_plain) {
   prof_end(c, LBM_PHASE_PARTICLES);
   int nf = 1 - c->fcur;
   prof_begin(c);
-  if (!pre) reset_flags(c, nf);
+  if (!pre) {
+    reset_flags(c, nf);
+    cudaMemsetAsync(c->fill.count, 0, sizeof(int32_t), c->stream);
+  }
+  launch_flags(c->g, pview(c), c->flags[nf], c->links, c->stream);
+  // the link lists on the aux stream (after the bounce-back stores and the
+  // overlap check there): the next bounce-back is their first reader, so they
+  // run beside the refill and the next stream + collide
+  cudaEventRecord(c->ev_aux_fork, c->stream);
+  cudaStreamWaitEvent(c->aux, c->ev_aux_fork, 0);
+  launch_link_lists(c->g, pview(c), c->links, c->status, c->f32 ? 1 : 0, c->aux);
+  cudaEventRecord(c->ev_links, c->aux);
+  c->links_pending = true;
+  prof_end(c, LBM_PHASE_LINKS);
+  prof_begin(c);
   if (c->store_pending) {
     cudaStreamWaitEvent(c->stream, c->ev_store, 0);
     c->store_pending = false;
   }
-  launch_links(c->g, pview(c), c->flags[nf], c->links, c->status, c->f32 ? 1 : 0, c->stream, true);
-  prof_end(c, LBM_PHASE_LINKS);
-  prof_begin(c);
   launch_filling<T>(c->g, pview(c), c->pp, c->ypglbp, c->wpp, c->omgpp, c->flags[nf],
                     c->flags[c->fcur], f_plain, c->fill, c->status, c->stream);
   prof_end(c, LBM_PHASE_FILLING);
@@ -628,6 +652,7 @@ void fused_step_t(lbm_ctx* c) {
   prof_end(c, LBM_PHASE_STREAM_COLLIDE);
   particle_prelude(c);
   if (c->particles_on) {
+    join_links(c);
     prof_begin(c);
     launch_bounce_back<T>(c->g, pview(c), fout, 1, c->flags[c->fcur], c->links, c->fHIp,
                           c->torqp, c->stream);
@@ -655,6 +680,7 @@ void unfused_step_t(lbm_ctx* c) {
                       mbuf<T>(c, 0), mbuf<T>(c, 1), mbuf<T>(c, 2), mbuf<T>(c, 3),
                       c->sums != LBM_SUMS_FLOAT, c->stream);
   if (c->particles_on) {
+    join_links(c);
     launch_bounce_back<T>(c->g, pview(c), fbuf<T>(c, c->cur), 0, c->flags[c->fcur], c->links,
                           c->fHIp, c->torqp, c->stream);
     launch_bounce_scatter<T>(c->g, pview(c), fbuf<T>(c, c->cur), 0, c->links, c->stream);
@@ -966,6 +992,7 @@ int lbm_create(const lbm_config* cfg, lbm_ctx** out) {
       cudaEventCreateWithFlags(&ctx->ev_aux_fork, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&ctx->ev_aux_join, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&ctx->ev_store, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&ctx->ev_links, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&ctx->ev_main, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&ctx->ev_forcing, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&ctx->ev_status, cudaEventDisableTiming) != cudaSuccess) {
@@ -1158,7 +1185,7 @@ int lbm_destroy(lbm_ctx* ctx) {
   if (ctx->side) cudaStreamDestroy(ctx->side);
   if (ctx->aux) cudaStreamDestroy(ctx->aux);
   for (cudaEvent_t e : {ctx->ev_main, ctx->ev_forcing, ctx->ev_status, ctx->ev_aux_fork,
-                        ctx->ev_aux_join, ctx->ev_store})
+                        ctx->ev_aux_join, ctx->ev_store, ctx->ev_links})
     if (e) cudaEventDestroy(e);
   delete ctx;
   return LBM_OK;
@@ -1835,6 +1862,7 @@ int lbm_beads_filling(lbm_ctx* ctx) {
   if (!ctx) return LBM_ERR_ARG;
   if (!ctx->particles_on) return LBM_OK;
   materialize_macro(ctx);
+  CK(cudaMemsetAsync(ctx->fill.count, 0, sizeof(int32_t), ctx->stream));
   if (ctx->f32)
     launch_filling<float>(ctx->g, pview(ctx), ctx->pp, ctx->ypglbp, ctx->wpp, ctx->omgpp,
                           ctx->flags[ctx->fcur], ctx->flags[1 - ctx->fcur],
@@ -1979,6 +2007,7 @@ int lbm_step(lbm_ctx* ctx, int nsteps) {
       if (ctx->f32) fused_step_t<float>(ctx); else fused_step_t<double>(ctx);
     }
   }
+  join_links(ctx);  // every other entry finds the lists complete
   CK(cudaGetLastError());
   if (ctx->particles_on || ctx->variant != LBM_VARIANT_DIRECT) {
     CK(cudaMemcpyAsync(ctx->status_host, ctx->status, sizeof(DevStatus), cudaMemcpyDeviceToHost,
@@ -2182,8 +2211,9 @@ struct lbm_batch {
   int max_npart = 0, max_nz = 0;
   long long max_reset = 0, max_rows = 0;
   bool stochastic = false;
-  cudaStream_t side = nullptr;
-  cudaEvent_t ev_side_all = nullptr;
+  cudaStream_t side = nullptr, aux = nullptr;
+  cudaEvent_t ev_side_all = nullptr, ev_aux_fork = nullptr, ev_aux_join = nullptr, ev_links = nullptr;
+  bool links_pending = false;  // the link lists run on aux until ev_links
   int64_t graph_kernels = 0;
   std::string err;
 };
@@ -2221,6 +2251,14 @@ bool same_phase(const lbm_batch* b) {
     if (!c->macro_derived || c->prefetched) return false;
   }
   return true;
+}
+
+// the link lists of the last step complete on the batch stream ("" or the error)
+std::string batch_join_links(lbm_batch* b) {
+  if (!b->links_pending) return "";
+  b->links_pending = false;
+  const cudaError_t e = cudaStreamWaitEvent(b->main, b->ev_links, 0);
+  return e == cudaSuccess ? "" : std::string("link lists: ") + cudaGetErrorString(e);
 }
 
 // One step of every box: the box's FORCING (prefetched during the previous
@@ -2292,8 +2330,10 @@ std::string batch_step_eager(lbm_batch* b) {
       c->batch_slot = slot;
     }
   }
+  if (!(err = batch_join_links(b)).empty()) return err;
   launch_particle_step_multi(b->d_parts[par], (int)b->ctx.size(), b->max_npart, b->max_reset,
-                             b->main);
+                             b->main, b->aux, b->ev_aux_fork, b->ev_aux_join, b->ev_links);
+  b->links_pending = b->max_npart > 0;
   if (!(err = chk(cudaGetLastError(), "particles", 0)).empty()) return err;
   if (b->stochastic &&
       !(err = chk(cudaStreamWaitEvent(b->main, b->ev_side_all, 0), "side join", 0)).empty())
@@ -2404,6 +2444,10 @@ int lbm_batch_create(lbm_ctx** ctxs, int n, lbm_batch** out) {
       cudaMalloc((void**)&b->d_parts[0], parts.size() * sizeof(BoxParticles)) != cudaSuccess ||
       cudaMalloc((void**)&b->d_forcing, forc.size() * sizeof(BoxForcing)) != cudaSuccess ||
       cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaStreamCreateWithFlags(&b->aux, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaEventCreateWithFlags(&b->ev_aux_fork, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&b->ev_aux_join, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&b->ev_links, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&b->ev_side_all, cudaEventDisableTiming) != cudaSuccess)
     rc = LBM_ERR_CUDA;
   if (!rc) b->d_parts[1] = b->d_parts[0] + n;
@@ -2442,6 +2486,7 @@ int lbm_batch_destroy(lbm_batch* b) {
   if (!b) return LBM_OK;
   if (b->main) cudaStreamSynchronize(b->main);
   if (b->side) cudaStreamSynchronize(b->side);
+  if (b->aux) cudaStreamSynchronize(b->aux);
   for (lbm_ctx* c : b->ctx) {
     if (c->side) cudaStreamSynchronize(c->side);
     if (c->stream) cudaStreamSynchronize(c->stream);
@@ -2466,6 +2511,9 @@ int lbm_batch_destroy(lbm_batch* b) {
   cudaFree(b->d_forcing);
   if (b->ev_side_all) cudaEventDestroy(b->ev_side_all);
   if (b->side) cudaStreamDestroy(b->side);
+  if (b->aux) cudaStreamDestroy(b->aux);
+  for (cudaEvent_t e : {b->ev_aux_fork, b->ev_aux_join, b->ev_links})
+    if (e) cudaEventDestroy(e);
   if (b->own_main && b->main) cudaStreamDestroy(b->main);
   delete b;
   return LBM_OK;
@@ -2496,6 +2544,8 @@ int lbm_batch_step(lbm_batch* b, int nsteps, int use_graph) {
         BK(cudaStreamBeginCapture(b->main, cudaStreamCaptureModeRelaxed));
         std::string err;
         for (int k = 0; k < kBatchCycle && err.empty(); ++k) err = batch_step_eager(b);
+        if (err.empty()) err = batch_join_links(b);
+        b->links_pending = false;
         cudaGraph_t gr = nullptr;
         cudaError_t ee = cudaStreamEndCapture(b->main, &gr);
         if (!err.empty() || ee != cudaSuccess) {
@@ -2518,9 +2568,10 @@ int lbm_batch_step(lbm_batch* b, int nsteps, int use_graph) {
       }
       nsteps -= kBatchCycle;
     } else {
-      const std::string err = batch_step_eager(b);
-      if (!err.empty()) return bfail(b, LBM_ERR_CUDA, "batch step: " + err);
+      std::string err = batch_step_eager(b);
       --nsteps;
+      if (err.empty() && (nsteps == 0 || (use_graph && nsteps >= kBatchCycle))) err = batch_join_links(b);
+      if (!err.empty()) return bfail(b, LBM_ERR_CUDA, "batch step: " + err);
     }
   }
   BK(cudaGetLastError());

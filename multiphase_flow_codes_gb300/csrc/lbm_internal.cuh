@@ -336,10 +336,16 @@ struct LinkSlab {
 };
 constexpr int kSweepBytes = 7 * 96;
 constexpr int kBounceSplit = 24;
+// beads_links: the sweeps (link_sweeps), the solid nodes of every particle
+// (flags and mask), its link list.  launch_links runs all three; a fused step
+// runs the sweeps with the move and the lists beside the refill.
 // alpha_fp32: link fractions in single precision (the FP32 population path)
 void launch_links(const Geometry& g, const ParticleView& pv, int32_t* isnodes,
-                  LinkSlab ls, DevStatus* st, int alpha_fp32, cudaStream_t s,
-                  bool sweeps_done = false);
+                  LinkSlab ls, DevStatus* st, int alpha_fp32, cudaStream_t s);
+void launch_flags(const Geometry& g, const ParticleView& pv, int32_t* isnodes, LinkSlab ls,
+                  cudaStream_t s);
+void launch_link_lists(const Geometry& g, const ParticleView& pv, LinkSlab ls, DevStatus* st,
+                       int alpha_fp32, cudaStream_t s);
 template <typename T>
 void launch_bounce_back(const Geometry& g, const ParticleView& pv, const T* f,
                         int pushed_layout, const int32_t* isnodes, LinkSlab ls,
@@ -401,9 +407,11 @@ struct BoxParticles {
   DevStatus* st;
 };
 // one launch per kernel of the particle step (bounce-back through refill)
-// for nb boxes of the array
+// for nb boxes of the array, on s and aux; the caller waits for ev_links
+// before the next particle step
 void launch_particle_step_multi(const BoxParticles* boxes, int nb, int max_npart,
-                                long long max_reset, cudaStream_t s);
+                                long long max_reset, cudaStream_t s, cudaStream_t aux,
+                                cudaEvent_t ev_fork, cudaEvent_t ev_join, cudaEvent_t ev_links);
 // FORCING of many boxes into table slot `slot`, keeping each box's state
 // before the update in `backup`
 struct BoxForcing {
@@ -419,6 +427,7 @@ struct BoxForcing {
 void launch_forcing_multi(const BoxForcing* boxes, int nb, int max_nz, long long max_rows,
                           int slot, cudaStream_t s);
 
+// (the refill list empty: fl.count zero)
 template <typename T>
 void launch_filling(const Geometry& g, const ParticleView& pv, const PartParams& pp,
                     const double* ypglbp, const double* wpp, const double* omgpp,

@@ -199,165 +199,43 @@ __device__ __noinline__ bool inside_fp64(int i, int j, int k, double xc, double 
   return (rr - rad2) <= 0.0;
 }
 
-__device__ __forceinline__ void k_links_body(int bx, int gx, Geometry g, ParticleView pv, int32_t* isnodes,
-                                              LinkSlab ls, DevStatus* st, int alpha_fp32) {
+// What beads_links' loop nest visits for one particle: candidate windows,
+// planes and rows with the image values in effect there, shared by the flag
+// and the link kernels.
+struct LinkSetup {
   using Scan = cub::BlockScan<int, PB>;
-  __shared__ typename Scan::TempStorage scan_tmp;
-  __shared__ int plane_k[MAXPLANES];
-  __shared__ double plane_z[MAXPLANES];
-  __shared__ double plane_zz[MAXPLANES];  // (k - 1/2) - zc of each plane
-  __shared__ double yval[3][MAXC];
-  __shared__ double yyv[3][MAXC];         // (j - 1/2) - yc per y candidate and start state
-  __shared__ float yyvf[3][MAXC];
-  __shared__ double xval[3][MAXC];
-  __shared__ float xofff[3][MAXC];  // (i - 1/2) - x centre per x candidate, FP64 then rounded
-  __shared__ int nplanes;
-  __shared__ int row_k[MAXROWS], row_j[MAXROWS];
-  __shared__ double row_z[MAXROWS], row_y[MAXROWS];
-  __shared__ float row_yy[MAXROWS], row_zz[MAXROWS];
-  __shared__ int nrows;
-  __shared__ int base;
-  __shared__ int fixed_ok;
-  __shared__ int near_rc[MAXNEAR];  // fluid nodes within reach: row << 8 | candidate
-  __shared__ int nnear;
+  typename Scan::TempStorage scan_tmp;
+  double par[5];  // radp2, rad2, x0, y0, z0
+  float parf[2];  // rad2 and the squared reach in FP32
+  int finite;
+  int fixed_ok;
+  int nplanes, nrows;
+  union {
+    struct {  // read by fill alone
+      double plane_z[MAXPLANES];
+      double plane_zz[MAXPLANES];  // (k - 1/2) - zc of each plane
+      double yval[3][MAXC];
+      double yyv[3][MAXC];         // (j - 1/2) - yc per y candidate and start state
+      float yyvf[3][MAXC];
+      int plane_k[MAXPLANES];
+    };
+    int16_t link_src[PB * 18];  // k_links: per link of the chunk, near node (local) << 5 | ipop
+  };
+  double xval[3][MAXC];
+  float xofff[3][MAXC];  // (i - 1/2) - x centre per x candidate, FP64 then rounded
+  int row_k[MAXROWS], row_j[MAXROWS];
+  double row_z[MAXROWS], row_y[MAXROWS];
+  float row_yy[MAXROWS], row_zz[MAXROWS];
+  // sweep event lists (link_sweeps): 0..2 the y sweep's start states (plane 0
+  // starts at y0, plane 1 at the end of plane 0's sweep, later planes at the
+  // end of that), 3..5 the x sweep's (rows likewise), 6 the single z sweep
+  SweepEv sev[7];
+  Cands cands[3];  // y, x, z
 
-  const int p = bx;
-  if (p >= pv.npart) return;
-  const bool channel = g.channel != 0;
-  const int tid = threadIdx.x;
-  // the block's FP64 constants, formed once (by thread 0) rather than by
-  // every warp: FP64 instructions are the scarce issue slots of this GPU
-  __shared__ double s_par[5];  // radp2, rad2, x0, y0, z0
-  __shared__ float s_parf[2];  // rad2 and the squared reach in FP32
-  __shared__ int s_finite;
-  if (tid == 0) {
-    nplanes = 0; nrows = 0; base = 0; fixed_ok = 1; nnear = 0;
-    const double rad = pv.rad;
-    s_par[0] = rad * 1.0 + 2.0;
-    s_par[1] = (rad * 1.0) * (rad * 1.0);
-    s_parf[0] = (float)s_par[1];
-    // only nodes within rad + sqrt(2) of the centre can be solid or own a link
-    s_parf[1] = (float)((rad + 1.5) * (rad + 1.5)) + 0.05f;
-    for (int a = 0; a < 3; ++a) s_par[2 + a] = pv.ypglb[3 * p + a] * 1.0;
-    s_finite = isfinite(s_par[2]) && isfinite(s_par[3]) && isfinite(s_par[4]);
-  }
-  __syncthreads();
-  const double radp2 = s_par[0], rad2 = s_par[1];
-  const float rad2f = s_parf[0], reachf = s_parf[1];
-  const double x0 = s_par[2], y0 = s_par[3], z0 = s_par[4];
-  if (!s_finite) {
-    if (tid == 0) {
-      ls.count[p] = 0;
-      raise_error(st, LBM_ERR_NONFINITE, p);
-    }
-    return;
-  }
-  // Sweep event lists (k_link_sweeps) for the start states of the y sweep
-  // (plane 0 starts at y0, plane 1 at Y1 = end of plane 0's sweep, later
-  // planes at Y2) and of the x sweep (rows likewise: x0, X1, X2), and for the
-  // single z sweep.
-  __shared__ SweepEv sev[7];  // 0..2: y states, 3..5: x states, 6: z
-  static_assert(sizeof(sev) % 4 == 0 && sizeof(sev) <= PB * 4, "one word a thread");
-  if (tid < (int)(sizeof(sev) / 4))
-    reinterpret_cast<int*>(sev)[tid] = reinterpret_cast<const int*>(
-        static_cast<const char*>(ls.sweeps) + (size_t)p * kSweepBytes)[tid];
-  if (tid == 0) {
-    const int32_t* ok = ls.sweep_ok + 3 * p;
-    if (!(ok[0] && ok[1] && ok[2])) fixed_ok = 0;
-  }
-  // candidate windows of the three axes, computed once for the block
-  __shared__ Cands cands[3];
-  if (tid == 0) cands[0] = make_cands(y0, g.ny, radp2, true);
-  else if (tid == 32) cands[1] = make_cands(x0, g.nx, radp2, !channel);
-  else if (tid == 64) cands[2] = make_cands(z0, g.nz, radp2, true);
-  __syncthreads();
-  const Cands& cy = cands[0];
-  const Cands& cx = cands[1];
-  const int ty = min(cy.total(), MAXC);
-  const int tx = min(cx.total(), MAXC);
-  for (int t = tid; t < 3 * MAXC; t += PB) {
-    int s = t / MAXC, c = t % MAXC;
-    if (c < ty) {
-      const double yc = sweep_value(sev[s], cy.at(c));
-      yval[s][c] = yc;
-      const double yy0 = ((double)cy.at(c) - 0.5) - yc;
-      yyv[s][c] = yy0;
-      yyvf[s][c] = (float)yy0;
-    }
-    if (c < tx) {
-      double v = channel ? x0 : sweep_value(sev[3 + s], cx.at(c));
-      xval[s][c] = v;
-      xofff[s][c] = (float)(((double)cx.at(c) - 0.5) - v);
-    }
-  }
-  if (tid == 0 && (cy.total() > MAXC || cx.total() > MAXC)) fixed_ok = 0;
-  __syncthreads();
+  __device__ __forceinline__ int tx() const { return min(cands[1].total(), MAXC); }
 
-  // ---- planes: k with |zz0| <= radp2, zc from the k-sweep starting at z0
-  const Cands& cz = cands[2];
-  int tz = cz.total();
-  for (int c0 = 0; c0 < tz; c0 += PB) {
-    int t = c0 + tid;
-    int k = -1;
-    double zc = 0.0, zz0 = 0.0;
-    bool take = false;
-    if (t < tz) {
-      k = cz.at(t);
-      zc = sweep_value(sev[6], k);
-      double zpnt = (double)k - 0.5;
-      zz0 = zpnt - zc;
-      take = fabs(zz0) <= radp2;
-    }
-    int pos, tot;
-    Scan(scan_tmp).ExclusiveSum(take ? 1 : 0, pos, tot);
-    __syncthreads();
-    if (take && nplanes + pos < MAXPLANES) {
-      plane_k[nplanes + pos] = k;
-      plane_z[nplanes + pos] = zc;
-      plane_zz[nplanes + pos] = zz0;
-    }
-    __syncthreads();
-    if (tid == 0) nplanes = min(nplanes + tot, MAXPLANES);
-    __syncthreads();
-  }
-
-  // ---- rows: per plane (in k order), j with the exact y condition
-  int tpairs = nplanes * ty;
-  for (int c0 = 0; c0 < tpairs; c0 += PB) {
-    int t = c0 + tid;
-    bool take = false;
-    int k = 0, j = 0, pi = 0, c = 0;
-    if (t < tpairs) {
-      // the offsets of the row's plane and y candidate come from the tables
-      // above (the same values; the FP64 work done once per plane and
-      // candidate rather than per pair)
-      pi = t / ty;
-      c = t - pi * ty;
-      j = cy.at(c);
-      k = plane_k[pi];
-      const double zz0 = plane_zz[pi], yy0 = yyv[min(pi, 2)][c];
-      take = channel ? (sqrt(yy0 * yy0 + zz0 * zz0) <= radp2) : (fabs(yy0) <= radp2);
-    }
-    int pos, tot;
-    Scan(scan_tmp).ExclusiveSum(take ? 1 : 0, pos, tot);
-    __syncthreads();
-    if (take && nrows + pos < MAXROWS) {
-      int w = nrows + pos;
-      row_k[w] = k; row_j[w] = j; row_z[w] = plane_z[pi]; row_y[w] = yval[min(pi, 2)][c];
-      row_yy[w] = yyvf[min(pi, 2)][c]; row_zz[w] = (float)plane_zz[pi];
-    }
-    __syncthreads();
-    if (tid == 0) nrows = min(nrows + tot, MAXROWS);
-    __syncthreads();
-  }
-
-  // ---- phase 1: nodes of every processed row within reach of the sphere;
-  // solid nodes are flagged, fluid ones kept (in row, then x order) for
-  // phase 2.  One thread per row; a block scan of the per-row counts places
-  // each row's nodes.
   // class of node (row r, x candidate ci): 0 out of reach, 1 solid, 2 fluid
-  auto node_class = [&](int r, int ci) -> int {
-    const int i = cx.at(ci);
+  __device__ __forceinline__ int node_class(int r, int ci, float rad2f, float reachf, double rad2) const {
     const float xxf = xofff[min(r, 2)][ci];
     const float yyf = row_yy[r], zzf = row_zz[r];
     const float rr0f = xxf * xxf + yyf * yyf + zzf * zzf;
@@ -365,41 +243,197 @@ __device__ __forceinline__ void k_links_body(int bx, int gx, Geometry g, Particl
     const float d0 = rr0f - rad2f;
     if (d0 < -kDecide) return 1;
     if (d0 > kDecide) return 2;
-    return inside_fp64(i, row_j[r], row_k[r], xval[min(r, 2)][ci], row_y[r], row_z[r], rad2) ? 1
-                                                                                             : 2;
-  };
-  for (int r0 = 0; r0 < nrows; r0 += PB) {
-    const int r = r0 + tid;
-    int cnt = 0;
-    if (r < nrows) {
-      const int j = row_j[r], k = row_k[r];
-      for (int ci = 0; ci < tx; ++ci) {
-        const int cl = node_class(r, ci);
-        if (cl == 1) {
-          const int i = cx.at(ci);
-          long long node = (long long)(i - 1) + (long long)g.nx * ((j - 1) + (long long)g.ny * (k - 1));
-          atomicMax(&isnodes[node], p);
-          uint32_t* mask = const_cast<uint32_t*>(solid_mask(isnodes, g));
-          atomicOr(&mask[((size_t)(k - 1) * g.ny + (j - 1)) * g.sw + ((i - 1) >> 5)],
-                   1u << ((i - 1) & 31));
-        } else if (cl == 2) {
-          ++cnt;
-        }
+    return inside_fp64(cands[1].at(ci), row_j[r], row_k[r], xval[min(r, 2)][ci], row_y[r], row_z[r], rad2) ? 1
+                                                                                                           : 2;
+  }
+
+  // fills the tables for particle p; false: its centre is not finite
+  __device__ __forceinline__ bool fill(int p, const Geometry& g, const ParticleView& pv, const LinkSlab& ls) {
+    const bool channel = g.channel != 0;
+    const int tid = threadIdx.x;
+    // the block's FP64 constants, formed once (by thread 0) rather than by
+    // every warp: FP64 instructions are the scarce issue slots of this GPU
+    if (tid == 0) {
+      nplanes = 0; nrows = 0; fixed_ok = 1;
+      const double rad = pv.rad;
+      par[0] = rad * 1.0 + 2.0;
+      par[1] = (rad * 1.0) * (rad * 1.0);
+      parf[0] = (float)par[1];
+      // only nodes within rad + sqrt(2) of the centre can be solid or own a link
+      parf[1] = (float)((rad + 1.5) * (rad + 1.5)) + 0.05f;
+      for (int a = 0; a < 3; ++a) par[2 + a] = pv.ypglb[3 * p + a] * 1.0;
+      finite = isfinite(par[2]) && isfinite(par[3]) && isfinite(par[4]);
+    }
+    static_assert(sizeof(sev) % 4 == 0 && sizeof(sev) <= PB * 4, "one word a thread");
+    if (tid < (int)(sizeof(sev) / 4))
+      reinterpret_cast<int*>(sev)[tid] = reinterpret_cast<const int*>(
+          static_cast<const char*>(ls.sweeps) + (size_t)p * kSweepBytes)[tid];
+    __syncthreads();
+    if (!finite) return false;
+    const double radp2 = par[0];
+    const double x0 = par[2], y0 = par[3], z0 = par[4];
+    // candidate windows of the three axes, computed once for the block
+    if (tid == 0) cands[0] = make_cands(y0, g.ny, radp2, true);
+    else if (tid == 32) cands[1] = make_cands(x0, g.nx, radp2, !channel);
+    else if (tid == 64) cands[2] = make_cands(z0, g.nz, radp2, true);
+    else if (tid == 96) {
+      const int32_t* ok = ls.sweep_ok + 3 * p;
+      if (!(ok[0] && ok[1] && ok[2])) fixed_ok = 0;
+    }
+    __syncthreads();
+    const Cands& cy = cands[0];
+    const Cands& cx = cands[1];
+    const int ty = min(cy.total(), MAXC);
+    const int ntx = tx();
+    for (int t = tid; t < 3 * MAXC; t += PB) {
+      int s = t / MAXC, c = t % MAXC;
+      if (c < ty) {
+        const double yc = sweep_value(sev[s], cy.at(c));
+        yval[s][c] = yc;
+        const double yy0 = ((double)cy.at(c) - 0.5) - yc;
+        yyv[s][c] = yy0;
+        yyvf[s][c] = (float)yy0;
+      }
+      if (c < ntx) {
+        double v = channel ? x0 : sweep_value(sev[3 + s], cx.at(c));
+        xval[s][c] = v;
+        xofff[s][c] = (float)(((double)cx.at(c) - 0.5) - v);
       }
     }
+    if (tid == 0 && (cy.total() > MAXC || cx.total() > MAXC)) fixed_ok = 0;
+
+    // ---- planes: k with |zz0| <= radp2, zc from the k-sweep starting at z0
+    const Cands& cz = cands[2];
+    int tz = cz.total();
+    for (int c0 = 0; c0 < tz; c0 += PB) {
+      int t = c0 + tid;
+      int k = -1;
+      double zc = 0.0, zz0 = 0.0;
+      bool take = false;
+      if (t < tz) {
+        k = cz.at(t);
+        zc = sweep_value(sev[6], k);
+        double zpnt = (double)k - 0.5;
+        zz0 = zpnt - zc;
+        take = fabs(zz0) <= radp2;
+      }
+      int pos, tot;
+      Scan(scan_tmp).ExclusiveSum(take ? 1 : 0, pos, tot);
+      __syncthreads();
+      if (take && nplanes + pos < MAXPLANES) {
+        plane_k[nplanes + pos] = k;
+        plane_z[nplanes + pos] = zc;
+        plane_zz[nplanes + pos] = zz0;
+      }
+      __syncthreads();
+      if (tid == 0) nplanes = min(nplanes + tot, MAXPLANES);
+      __syncthreads();
+    }
+
+    // ---- rows: per plane (in k order), j with the exact y condition
+    int tpairs = nplanes * ty;
+    for (int c0 = 0; c0 < tpairs; c0 += PB) {
+      int t = c0 + tid;
+      bool take = false;
+      int k = 0, j = 0, pi = 0, c = 0;
+      if (t < tpairs) {
+        // the offsets of the row's plane and y candidate come from the tables
+        // above (the same values; the FP64 work done once per plane and
+        // candidate rather than per pair)
+        pi = t / ty;
+        c = t - pi * ty;
+        j = cy.at(c);
+        k = plane_k[pi];
+        const double zz0 = plane_zz[pi], yy0 = yyv[min(pi, 2)][c];
+        take = channel ? (sqrt(yy0 * yy0 + zz0 * zz0) <= radp2) : (fabs(yy0) <= radp2);
+      }
+      int pos, tot;
+      Scan(scan_tmp).ExclusiveSum(take ? 1 : 0, pos, tot);
+      __syncthreads();
+      if (take && nrows + pos < MAXROWS) {
+        int w = nrows + pos;
+        row_k[w] = k; row_j[w] = j; row_z[w] = plane_z[pi]; row_y[w] = yval[min(pi, 2)][c];
+        row_yy[w] = yyvf[min(pi, 2)][c]; row_zz[w] = (float)plane_zz[pi];
+      }
+      __syncthreads();
+      if (tid == 0) nrows = min(nrows + tot, MAXROWS);
+      __syncthreads();
+    }
+    return true;
+  }
+};
+
+// The solid nodes of one particle per block: all that the refill, and with it
+// the next stream + collide, needs of beads_links.  A thread takes node after
+// node of all rows.
+__device__ __forceinline__ void k_flags_body(int p, const Geometry& g, const ParticleView& pv, int32_t* isnodes,
+                                              const LinkSlab& ls) {
+  __shared__ LinkSetup S;
+  if (p >= pv.npart) return;
+  if (!S.fill(p, g, pv, ls)) return;
+  const Cands& cx = S.cands[1];
+  const int tx = S.tx(), total = S.nrows * tx;
+  const float rad2f = S.parf[0], reachf = S.parf[1];
+  const double rad2 = S.par[1];
+  uint32_t* mask = const_cast<uint32_t*>(solid_mask(isnodes, g));
+  for (int t = threadIdx.x; t < total; t += PB) {
+    const int r = t / tx, ci = t - r * tx;
+    if (S.node_class(r, ci, rad2f, reachf, rad2) != 1) continue;
+    const int i = cx.at(ci), row = (S.row_k[r] - 1) * g.ny + (S.row_j[r] - 1);
+    atomicMax(&isnodes[(long long)row * g.nx + (i - 1)], p);
+    atomicOr(&mask[(size_t)row * g.sw + ((i - 1) >> 5)], 1u << ((i - 1) & 31));
+  }
+}
+__global__ void __launch_bounds__(PB) k_flags(Geometry g, ParticleView pv, int32_t* isnodes, LinkSlab ls) {
+  k_flags_body(blockIdx.x, g, pv, isnodes, ls);
+}
+
+// The boundary links of one particle per block and what the bounce-back
+// needs of each: the next bounce-back is their first reader, so this runs
+// beside the refill and the next stream + collide.
+__device__ __forceinline__ void k_links_body(int p, const Geometry& g, const ParticleView& pv,
+                                              const LinkSlab& ls, DevStatus* st, int alpha_fp32) {
+  __shared__ LinkSetup S;
+  __shared__ int base;
+  __shared__ int near_rc[MAXNEAR];  // fluid nodes within reach: row << 8 | candidate
+  __shared__ int nnear;
+  using Scan = LinkSetup::Scan;
+  if (p >= pv.npart) return;
+  const int tid = threadIdx.x;
+  if (tid == 0) { base = 0; nnear = 0; }
+  if (!S.fill(p, g, pv, ls)) {
+    if (tid == 0) {
+      ls.count[p] = 0;
+      raise_error(st, LBM_ERR_NONFINITE, p);
+    }
+    return;
+  }
+  const double rad2 = S.par[1];
+  const float rad2f = S.parf[0], reachf = S.parf[1];
+  const Cands& cx = S.cands[1];
+  const int tx = S.tx();
+
+  // ---- phase 1: the fluid nodes of every processed row within reach of the
+  // sphere (in row, then x order).  One thread per row; a block scan of the
+  // per-row counts places each row's nodes.
+  for (int r0 = 0; r0 < S.nrows; r0 += PB) {
+    const int r = r0 + tid;
+    int cnt = 0;
+    if (r < S.nrows)
+      for (int ci = 0; ci < tx; ++ci) cnt += S.node_class(r, ci, rad2f, reachf, rad2) == 2;
     int pos, tot;
-    Scan(scan_tmp).ExclusiveSum(cnt, pos, tot);
+    Scan(S.scan_tmp).ExclusiveSum(cnt, pos, tot);
     if (cnt) {
       int w = nnear + pos;
       for (int ci = 0; ci < tx; ++ci)
-        if (node_class(r, ci) == 2) {
+        if (S.node_class(r, ci, rad2f, reachf, rad2) == 2) {
           if (w < MAXNEAR) near_rc[w] = (r << 8) | ci;
           ++w;
         }
     }
     __syncthreads();
     if (tid == 0) {
-      if (nnear + tot > MAXNEAR) fixed_ok = 0;
+      if (nnear + tot > MAXNEAR) S.fixed_ok = 0;
       nnear = min(nnear + tot, MAXNEAR);
     }
     __syncthreads();
@@ -416,7 +450,6 @@ __device__ __forceinline__ void k_links_body(int bx, int gx, Geometry g, Particl
   constexpr int PER_LANE = (NCNT + 31) / 32;
   __shared__ int woff[NCNT];
   __shared__ int chunk_links;
-  __shared__ int16_t link_src[PB * 18];  // per link of the chunk: near node (local) << 5 | ipop
   const int warp = tid >> 5, lane = tid & 31;
   const unsigned lane_lt = (1u << lane) - 1u;
   int32_t* code = ls.code + (long long)p * ls.cap;
@@ -432,9 +465,9 @@ __device__ __forceinline__ void k_links_body(int bx, int gx, Geometry g, Particl
       r = rc >> 8;
       ci = rc & 255;
       i = cx.at(ci);
-      xxf = xofff[min(r, 2)][ci];
-      yyf = row_yy[r];
-      zzf = row_zz[r];
+      xxf = S.xofff[min(r, 2)][ci];
+      yyf = S.row_yy[r];
+      zzf = S.row_zz[r];
 #pragma unroll
       for (int ipop = 1; ipop < NPOP; ++ipop) {
         const float ax = xxf + (float)cix(ipop), ay = yyf + (float)ciy(ipop), az = zzf + (float)ciz(ipop);
@@ -443,8 +476,8 @@ __device__ __forceinline__ void k_links_body(int bx, int gx, Geometry g, Particl
         if (d1 < -kDecide) link = true;
         else if (d1 > kDecide) link = false;
         else
-          link = inside_fp64(i + cix(ipop), row_j[r] + ciy(ipop), row_k[r] + ciz(ipop),
-                             xval[min(r, 2)][ci], row_y[r], row_z[r], rad2);
+          link = inside_fp64(i + cix(ipop), S.row_j[r] + ciy(ipop), S.row_k[r] + ciz(ipop),
+                             S.xval[min(r, 2)][ci], S.row_y[r], S.row_z[r], rad2);
         if (link) mask |= 1u << ipop;
       }
     }
@@ -480,7 +513,7 @@ __device__ __forceinline__ void k_links_body(int bx, int gx, Geometry g, Particl
     }
     __syncthreads();
     {
-      const int j = row_j[r], k = row_k[r];
+      const int j = S.row_j[r], k = S.row_k[r];
       const long long node =
           (long long)(i - 1) + (long long)g.nx * ((j - 1) + (long long)g.ny * (k - 1));
 #pragma unroll 1
@@ -490,7 +523,7 @@ __device__ __forceinline__ void k_links_body(int bx, int gx, Geometry g, Particl
         const unsigned bal = __ballot_sync(0xffffffffu, has);
         if (!has) continue;
         const int l = woff[q * NW + warp] + __popc(bal & lane_lt);
-        link_src[l] = (int16_t)((tid << 5) | ipop);
+        S.link_src[l] = (int16_t)((tid << 5) | ipop);
         if (base + l < ls.cap) code[base + l] = (int32_t)(node * 32 + ipop);
       }
     }
@@ -499,7 +532,7 @@ __device__ __forceinline__ void k_links_body(int bx, int gx, Geometry g, Particl
     for (int l = tid; l < chunk_links; l += PB) {
       const int w = base + l;
       if (w >= ls.cap) break;
-      const int src = link_src[l];
+      const int src = S.link_src[l];
       const int ipop = src & 31;
       const int rc = near_rc[n0 + (src >> 5)];
       const int lr = rc >> 8, lci = rc & 255;
@@ -510,8 +543,8 @@ __device__ __forceinline__ void k_links_body(int bx, int gx, Geometry g, Particl
       // bb = x1.(x0 - x1) = -x1.c taken exactly: the same root without the
       // cancellation in the reference's aa and without divisions
       if (alpha_fp32 == 1) {
-        const float xf = xofff[min(lr, 2)][lci] + (float)ix;
-        const float yf = row_yy[lr] + (float)iy, zf = row_zz[lr] + (float)iz;
+        const float xf = S.xofff[min(lr, 2)][lci] + (float)ix;
+        const float yf = S.row_yy[lr] + (float)iy, zf = S.row_zz[lr] + (float)iz;
         const float cc = xf * xf + yf * yf + zf * zf - rad2f;
         const float bb = -(xf * (float)ix + yf * (float)iy + zf * (float)iz);
         const float a0 = diag ? 0.5f * bb : bb;
@@ -521,10 +554,10 @@ __device__ __forceinline__ void k_links_body(int bx, int gx, Geometry g, Particl
       } else {
         // the components of c are +-1 or 0: c . x1 is selects and one add
         auto pick = [](int c, double v) { return flip_if(c < 0, v); };
-        const int lj = row_j[lr], lk = row_k[lr];
-        const double xx1 = (double)(li + ix) - 0.5 - xval[min(lr, 2)][lci];
-        const double yy1 = (double)(lj + iy) - 0.5 - row_y[lr];
-        const double zz1 = (double)(lk + iz) - 0.5 - row_z[lr];
+        const int lj = S.row_j[lr], lk = S.row_k[lr];
+        const double xx1 = (double)(li + ix) - 0.5 - S.xval[min(lr, 2)][lci];
+        const double yy1 = (double)(lj + iy) - 0.5 - S.row_y[lr];
+        const double zz1 = (double)(lk + iz) - 0.5 - S.row_z[lr];
         double bb;
         if (ix == 0) bb = iy == 0 ? pick(iz, zz1) : (iz == 0 ? pick(iy, yy1) : pick(iy, yy1) + pick(iz, zz1));
         else bb = iy != 0 ? pick(ix, xx1) + pick(iy, yy1)
@@ -548,13 +581,13 @@ __device__ __forceinline__ void k_links_body(int bx, int gx, Geometry g, Particl
   if (tid == 0) {
     ls.count[p] = min(base, ls.cap);
     if (base > ls.cap) raise_error(st, LBM_ERR_CAPACITY, p);
-    if (nplanes >= MAXPLANES || nrows >= MAXROWS) raise_error(st, LBM_ERR_CAPACITY, p);
-    if (!fixed_ok) raise_error(st, LBM_ERR_STATE, p);
+    if (S.nplanes >= MAXPLANES || S.nrows >= MAXROWS) raise_error(st, LBM_ERR_CAPACITY, p);
+    if (!S.fixed_ok) raise_error(st, LBM_ERR_STATE, p);
   }
 }
-__global__ void __launch_bounds__(PB) k_links(Geometry g, ParticleView pv, int32_t* isnodes,
-                                              LinkSlab ls, DevStatus* st, int alpha_fp32) {
-  k_links_body(blockIdx.x, gridDim.x, g, pv, isnodes, ls, st, alpha_fp32);
+__global__ void __launch_bounds__(PB) k_links(Geometry g, ParticleView pv, LinkSlab ls, DevStatus* st,
+                                              int alpha_fp32) {
+  k_links_body(blockIdx.x, g, pv, ls, st, alpha_fp32);
 }
 
 // running sum: plain FP64, or FP32 with Kahan compensation (FP32 path)
@@ -1459,12 +1492,22 @@ int sm_count() {
   return sms;
 }
 
-void launch_links(const Geometry& g, const ParticleView& pv, int32_t* isnodes, LinkSlab ls,
-                  DevStatus* st, int alpha_fp32, cudaStream_t s, bool sweeps_done) {
+void launch_flags(const Geometry& g, const ParticleView& pv, int32_t* isnodes, LinkSlab ls,
+                  cudaStream_t s) {
   if (pv.npart <= 0) return;
-  if (!sweeps_done)
-    { k_link_sweeps<<<(3 * pv.npart + kSmallBlock - 1) / kSmallBlock, kSmallBlock, 0, s>>>(g, pv, ls); count_launch(); }
-  { k_links<<<pv.npart, PB, 0, s>>>(g, pv, isnodes, ls, st, alpha_fp32); count_launch(); }
+  { k_flags<<<pv.npart, PB, 0, s>>>(g, pv, isnodes, ls); count_launch(); }
+}
+void launch_link_lists(const Geometry& g, const ParticleView& pv, LinkSlab ls, DevStatus* st,
+                       int alpha_fp32, cudaStream_t s) {
+  if (pv.npart <= 0) return;
+  { k_links<<<pv.npart, PB, 0, s>>>(g, pv, ls, st, alpha_fp32); count_launch(); }
+}
+void launch_links(const Geometry& g, const ParticleView& pv, int32_t* isnodes, LinkSlab ls,
+                  DevStatus* st, int alpha_fp32, cudaStream_t s) {
+  if (pv.npart <= 0) return;
+  { k_link_sweeps<<<(3 * pv.npart + kSmallBlock - 1) / kSmallBlock, kSmallBlock, 0, s>>>(g, pv, ls); count_launch(); }
+  launch_flags(g, pv, isnodes, ls, s);
+  launch_link_lists(g, pv, ls, st, alpha_fp32, s);
 }
 
 // Blocks that share a particle's bounce-back (FP64): as many as take one
@@ -1541,7 +1584,6 @@ void launch_filling(const Geometry& g, const ParticleView& pv, const PartParams&
                     const int32_t* isnodes, const int32_t* isnodes0, T* f, FillList fl,
                     DevStatus* st, cudaStream_t s) {
   if (pv.npart <= 0) return;
-  cudaMemsetAsync(fl.count, 0, sizeof(int), s);
   { k_fill_detect<<<pv.npart, PB, 0, s>>>(g, pv, pp, ypglbp, isnodes, isnodes0, fl, st); count_launch(); }
   // eight blocks of four warps per SM: one refill event per warp for up to
   // 32 events an SM (the events' serial FP64 chains then run side by side)
@@ -1594,9 +1636,13 @@ __global__ void k_reset_multi(const BoxParticles* boxes) {
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) *B.fl.count = 0;
 }
+__global__ void __launch_bounds__(PB) k_flags_multi(const BoxParticles* boxes) {
+  BOX_OR_RETURN(B.pv.npart)
+  k_flags_body(blockIdx.x, B.g, B.pv, B.flags_next, B.ls);
+}
 __global__ void __launch_bounds__(PB) k_links_multi(const BoxParticles* boxes) {
   BOX_OR_RETURN(B.pv.npart)
-  k_links_body(blockIdx.x, nblk, B.g, B.pv, B.flags_next, B.ls, B.st, 1);
+  k_links_body(blockIdx.x, B.g, B.pv, B.ls, B.st, 1);
 }
 __global__ void __launch_bounds__(PB) k_fill_detect_multi(const BoxParticles* boxes) {
   BOX_OR_RETURN(B.pv.npart)
@@ -1613,18 +1659,40 @@ __global__ void __launch_bounds__(128) k_fill_events_multi(const BoxParticles* b
 
 }  // namespace
 
+// The particle step on s; what no kernel of s waits for at once runs on aux,
+// as for a single box: the flag reset and beads_lubforce beside the
+// bounce-back (forked before it by ev_fork), the bounce-back stores and the
+// overlap check beside move and flags, the link lists (ev_links) beside the
+// refill and the next stream + collide.
 void launch_particle_step_multi(const BoxParticles* boxes, int nb, int max_npart,
-                                long long max_reset, cudaStream_t s) {
+                                long long max_reset, cudaStream_t s, cudaStream_t aux,
+                                cudaEvent_t ev_fork, cudaEvent_t ev_join, cudaEvent_t ev_links) {
   if (nb <= 0 || max_npart <= 0) return;
   auto grid = [&](long long blocks) { return dim3((unsigned)(blocks > 0 ? blocks : 1), nb); };
-  k_bounce_multi<<<grid(max_npart), bounce_threads<float>(), 0, s>>>(boxes); count_launch();
-  k_bounce_store_multi<<<grid(max_npart), PB, 0, s>>>(boxes); count_launch();
-  k_lubforce_multi<<<grid((max_npart * 32 + 127) / 128), 128, 0, s>>>(boxes); count_launch();
-  k_move_wrap_sweeps_multi<<<grid((3 * max_npart + kSmallBlock - 1) / kSmallBlock), kSmallBlock, 0, s>>>(boxes); count_launch();
-  k_overlap_multi<<<grid((max_npart * 32 + 127) / 128), 128, 0, s>>>(boxes); count_launch();
+  auto fork = [&]() {
+    cudaEventRecord(ev_fork, s);
+    cudaStreamWaitEvent(aux, ev_fork, 0);
+  };
+  auto join = [&]() {
+    cudaEventRecord(ev_join, aux);
+    cudaStreamWaitEvent(s, ev_join, 0);
+  };
+  fork();
   const long long rb = (max_reset + 256 * 8 - 1) / (256 * 8);
-  k_reset_multi<<<grid(rb < 1024 ? rb : 1024), 256, 0, s>>>(boxes); count_launch();
-  k_links_multi<<<grid(max_npart), PB, 0, s>>>(boxes); count_launch();
+  k_reset_multi<<<grid(rb < 1024 ? rb : 1024), 256, 0, aux>>>(boxes); count_launch();
+  k_lubforce_multi<<<grid((max_npart * 32 + 127) / 128), 128, 0, aux>>>(boxes); count_launch();
+  k_bounce_multi<<<grid(max_npart), bounce_threads<float>(), 0, s>>>(boxes); count_launch();
+  join();
+  fork();
+  k_bounce_store_multi<<<grid(max_npart), PB, 0, aux>>>(boxes); count_launch();
+  k_move_wrap_sweeps_multi<<<grid((3 * max_npart + kSmallBlock - 1) / kSmallBlock), kSmallBlock, 0, s>>>(boxes); count_launch();
+  fork();
+  k_overlap_multi<<<grid((max_npart * 32 + 127) / 128), 128, 0, aux>>>(boxes); count_launch();
+  k_flags_multi<<<grid(max_npart), PB, 0, s>>>(boxes); count_launch();
+  join();
+  fork();
+  k_links_multi<<<grid(max_npart), PB, 0, aux>>>(boxes); count_launch();
+  cudaEventRecord(ev_links, aux);
   k_fill_detect_multi<<<grid(max_npart), PB, 0, s>>>(boxes); count_launch();
   k_fill_events_multi<<<grid(kFillBlocks), 128, 0, s>>>(boxes); count_launch();
 }
