@@ -52,6 +52,7 @@ struct lbm_ctx {
   // the link lists of a fused step run on aux until ev_links (join_links)
   cudaEvent_t ev_links = nullptr;
   bool links_pending = false;
+  bool links_prep = false;  // the link lists hold the bounce-back's gathers too
   bool aux_pending = false;
   bool store_pending = false;  // the bounce-back stores run on aux until ev_store
   bool prefetched = false;
@@ -506,6 +507,13 @@ void join_links(lbm_ctx* c) {
   c->links_pending = false;
 }
 
+// whether link lists are built with the bounce-back's gathers (FP32, few spheres)
+bool want_prep(const lbm_ctx* c) { return c->f32 && c->npart <= kPrepParticles; }
+void links_now(lbm_ctx* c, int32_t* flags) {
+  c->links_prep = want_prep(c);
+  launch_links(c->g, pview(c), flags, c->links, c->status, c->f32 ? 1 : 0, c->links_prep, c->stream);
+}
+
 // The part of the particle step that reads no post-collision populations:
 // the reset of the flag buffer beads_links fills next (last read by the
 // previous step's beads_filling) and of the refill list, and beads_lubforce
@@ -561,7 +569,9 @@ void particle_phase(lbm_ctx* c, T* f_plain) {
   // run beside the refill and the next stream + collide
   cudaEventRecord(c->ev_aux_fork, c->stream);
   cudaStreamWaitEvent(c->aux, c->ev_aux_fork, 0);
-  launch_link_lists(c->g, pview(c), c->links, c->status, c->f32 ? 1 : 0, c->aux);
+  c->links_prep = want_prep(c);
+  launch_link_lists(c->g, pview(c), c->flags[nf], c->links, c->status, c->f32 ? 1 : 0, c->links_prep,
+                    c->aux);
   cudaEventRecord(c->ev_links, c->aux);
   c->links_pending = true;
   prof_end(c, LBM_PHASE_LINKS);
@@ -655,7 +665,7 @@ void fused_step_t(lbm_ctx* c) {
     join_links(c);
     prof_begin(c);
     launch_bounce_back<T>(c->g, pview(c), fout, 1, c->flags[c->fcur], c->links, c->fHIp,
-                          c->torqp, c->stream);
+                          c->torqp, c->links_prep, c->stream);
     prof_end(c, LBM_PHASE_BOUNCE);
     bounce_store_aux<T>(c, fout);
     particle_phase<T>(c, fout);
@@ -682,7 +692,7 @@ void unfused_step_t(lbm_ctx* c) {
   if (c->particles_on) {
     join_links(c);
     launch_bounce_back<T>(c->g, pview(c), fbuf<T>(c, c->cur), 0, c->flags[c->fcur], c->links,
-                          c->fHIp, c->torqp, c->stream);
+                          c->fHIp, c->torqp, c->links_prep, c->stream);
     launch_bounce_scatter<T>(c->g, pview(c), fbuf<T>(c, c->cur), 0, c->links, c->stream);
   }
   launch_streaming<T>(c->g, fbuf<T>(c, c->cur), fbuf<T>(c, 1 - c->cur), c->stream);
@@ -715,6 +725,7 @@ uint64_t footprint(const lbm_config& c, int64_t* cap_out) {
   if (cap_out) *cap_out = cap;
   b += np * 15 * 3 * 8;
   b += np * (uint64_t)cap * (4 + 8 + 8) + np * 4;
+  if (es == 4) b += std::min<uint64_t>(np, kPrepParticles) * (uint64_t)cap * (3 + 6) * 4;
   b += np * (kSweepBytes + 3 * 4);                       // nearest-image sweeps
   b += np * ((es == 8 ? 6ull * kBounceSplit * 8 : 0) + 4);  // bounce-back partial sums
   if (np > 0) b += 2ull * std::max<uint64_t>(4096, 256 * np) * 4 + 4;  // refill list
@@ -1038,6 +1049,11 @@ int lbm_create(const lbm_config* cfg, lbm_ctx** out) {
     al((void**)&ctx->links.code, (size_t)ctx->npmax * cap * sizeof(int32_t));
     al((void**)&ctx->links.alpha, (size_t)ctx->npmax * cap * sizeof(double));
     al((void**)&ctx->links.f9, (size_t)ctx->npmax * cap * sizeof(double));
+    if (ctx->f32) {
+      const size_t np = std::min(ctx->npmax, kPrepParticles);
+      al((void**)&ctx->links.gather, np * cap * 3 * sizeof(int32_t));
+      al((void**)&ctx->links.coef, np * cap * 6 * sizeof(float));
+    }
     al((void**)&ctx->links.count, (size_t)ctx->npmax * sizeof(int32_t));
     al(&ctx->links.sweeps, (size_t)ctx->npmax * kSweepBytes);
     al((void**)&ctx->links.sweep_ok, (size_t)ctx->npmax * 3 * sizeof(int32_t));
@@ -1173,7 +1189,8 @@ int lbm_destroy(lbm_ctx* ctx) {
                   ctx->rowtab[0], ctx->rowtab[1],
                   ctx->rowtab[2], ctx->pbuf, ctx->first_move, ctx->links.code,
                   ctx->links.alpha, ctx->links.f9, ctx->links.count, ctx->links.sweeps,
-                  ctx->links.sweep_ok, ctx->links.bsum, ctx->links.bdone, ctx->fill.node,
+                  ctx->links.sweep_ok, ctx->links.bsum, ctx->links.bdone,
+                  ctx->links.gather, ctx->links.coef, ctx->fill.node,
                   ctx->fill.part, ctx->fill.count, ctx->fcache, ctx->xtw_i,
                   ctx->rowtab_i[0], ctx->rowtab_i[1], ctx->rowtab_i[2]};
   for (void* p : ptrs)
@@ -1590,7 +1607,7 @@ int lbm_upload_particles(lbm_ctx* ctx, int npart, const double* ypglb, const dou
   CK(reset_flags(ctx, 0));
   CK(reset_flags(ctx, 1));
   ctx->particles_on = npart > 0;
-  if (npart > 0) launch_links(ctx->g, pview(ctx), ctx->flags[ctx->fcur], ctx->links, ctx->status, ctx->f32 ? 1 : 0, ctx->stream);
+  if (npart > 0) links_now(ctx, ctx->flags[ctx->fcur]);
   CK(cudaGetLastError());
   return check_status(ctx);
 }
@@ -1667,8 +1684,7 @@ int lbm_particle_state(lbm_ctx* ctx, int dir, int npart, double* state, int32_t*
   CK(reset_flags(ctx, 1));
   ctx->particles_on = npart > 0;
   if (npart > 0)
-    launch_links(ctx->g, pview(ctx), ctx->flags[ctx->fcur], ctx->links, ctx->status, ctx->f32 ? 1 : 0,
-                 ctx->stream);
+    links_now(ctx, ctx->flags[ctx->fcur]);
   CK(cudaGetLastError());
   return check_status(ctx);
 }
@@ -1798,11 +1814,11 @@ int lbm_beads_collision(lbm_ctx* ctx) {
   materialize_macro(ctx);
   if (ctx->f32) {
     launch_bounce_back<float>(ctx->g, pview(ctx), fbuf<float>(ctx, ctx->cur), 0, ctx->flags[ctx->fcur],
-                              ctx->links, ctx->fHIp, ctx->torqp, ctx->stream);
+                              ctx->links, ctx->fHIp, ctx->torqp, ctx->links_prep, ctx->stream);
     launch_bounce_scatter<float>(ctx->g, pview(ctx), fbuf<float>(ctx, ctx->cur), 0, ctx->links, ctx->stream);
   } else {
     launch_bounce_back<double>(ctx->g, pview(ctx), fbuf<double>(ctx, ctx->cur), 0, ctx->flags[ctx->fcur],
-                               ctx->links, ctx->fHIp, ctx->torqp, ctx->stream);
+                               ctx->links, ctx->fHIp, ctx->torqp, ctx->links_prep, ctx->stream);
     launch_bounce_scatter<double>(ctx->g, pview(ctx), fbuf<double>(ctx, ctx->cur), 0, ctx->links, ctx->stream);
   }
   ctx->macro_derived = false;
@@ -1852,7 +1868,7 @@ int lbm_beads_links(lbm_ctx* ctx) {
   if (!ctx->particles_on) return LBM_OK;
   int nf = 1 - ctx->fcur;
   CK(reset_flags(ctx, nf));
-  launch_links(ctx->g, pview(ctx), ctx->flags[nf], ctx->links, ctx->status, ctx->f32 ? 1 : 0, ctx->stream);
+  links_now(ctx, ctx->flags[nf]);
   ctx->fcur = nf;
   CK(cudaGetLastError());
   return check_status(ctx);
@@ -2214,6 +2230,8 @@ struct lbm_batch {
   cudaStream_t side = nullptr, aux = nullptr;
   cudaEvent_t ev_side_all = nullptr, ev_aux_fork = nullptr, ev_aux_join = nullptr, ev_links = nullptr;
   bool links_pending = false;  // the link lists run on aux until ev_links
+  // the boxes' link lists hold the bounce-back's gathers (few spheres in all)
+  bool prep = false;
   int64_t graph_kernels = 0;
   std::string err;
 };
@@ -2331,7 +2349,7 @@ std::string batch_step_eager(lbm_batch* b) {
     }
   }
   if (!(err = batch_join_links(b)).empty()) return err;
-  launch_particle_step_multi(b->d_parts[par], (int)b->ctx.size(), b->max_npart, b->max_reset,
+  launch_particle_step_multi(b->d_parts[par], (int)b->ctx.size(), b->max_npart, b->max_reset, b->prep,
                              b->main, b->aux, b->ev_aux_fork, b->ev_aux_join, b->ev_links);
   b->links_pending = b->max_npart > 0;
   if (!(err = chk(cudaGetLastError(), "particles", 0)).empty()) return err;
@@ -2344,6 +2362,7 @@ std::string batch_step_eager(lbm_batch* b) {
     c->fmacro = c->latest;
     c->macro_pending = true;
     c->macro_derived = true;
+    c->links_prep = b->prep;
   }
   return "";
 }
@@ -2378,6 +2397,16 @@ int lbm_batch_create(lbm_ctx** ctxs, int n, lbm_batch** out) {
     c->in_batch = true;
     c->fcache_slot = -1;
   }
+  // few spheres in all: lists with the gathers, also those built before
+  long long spheres = 0;
+  for (lbm_ctx* c : b->ctx) spheres += c->particles_on ? c->npart : 0;
+  b->prep = spheres > 0 && spheres <= kPrepParticles;
+  for (lbm_ctx* c : b->ctx)
+    if (b->prep && c->particles_on && !c->links_prep) {
+      launch_link_lists(c->g, pview(c), c->flags[c->fcur], c->links, c->status, 1, true, c->stream);
+      cudaStreamSynchronize(c->stream);
+      c->links_prep = true;
+    }
   // boxes and tasks
   std::vector<BatchBox> boxes(n);
   std::vector<BatchTask> tasks;

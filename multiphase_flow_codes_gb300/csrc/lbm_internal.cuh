@@ -326,6 +326,12 @@ struct LinkSlab {
   double* f9;
   int32_t* count;
   int cap;
+  // FP32 with up to kPrepParticles spheres, per link, for the bounce-back of a
+  // fused step: the elements of the pushed populations that ff1, ff2, ff3 are
+  // (-1: none) and c1, c2, c3 and the lever arm (ex, ey, ez); each particle's
+  // slab holds 3 and 6 runs of cap
+  int32_t* gather;
+  float* coef;
   void* sweeps;      // per particle: nearest-image sweep events of the 3 axes (kSweepBytes)
   int32_t* sweep_ok; // per particle and axis: 1 if the sweep reached its fixed point
   // a particle's bounce-back over several blocks (k_bounce): FP64, their
@@ -336,20 +342,23 @@ struct LinkSlab {
 };
 constexpr int kSweepBytes = 7 * 96;
 constexpr int kBounceSplit = 24;
+constexpr int kPrepParticles = 304;  // two spheres an SM
 // beads_links: the sweeps (link_sweeps), the solid nodes of every particle
 // (flags and mask), its link list.  launch_links runs all three; a fused step
 // runs the sweeps with the move and the lists beside the refill.
-// alpha_fp32: link fractions in single precision (the FP32 population path)
+// alpha_fp32: link fractions in single precision (the FP32 population path);
+// prep (FP32 only): with the bounce-back's gathers and coefficients, for
+// launch_bounce_back's prep
 void launch_links(const Geometry& g, const ParticleView& pv, int32_t* isnodes,
-                  LinkSlab ls, DevStatus* st, int alpha_fp32, cudaStream_t s);
+                  LinkSlab ls, DevStatus* st, int alpha_fp32, bool prep, cudaStream_t s);
 void launch_flags(const Geometry& g, const ParticleView& pv, int32_t* isnodes, LinkSlab ls,
                   cudaStream_t s);
-void launch_link_lists(const Geometry& g, const ParticleView& pv, LinkSlab ls, DevStatus* st,
-                       int alpha_fp32, cudaStream_t s);
+void launch_link_lists(const Geometry& g, const ParticleView& pv, const int32_t* isnodes, LinkSlab ls,
+                       DevStatus* st, int alpha_fp32, bool prep, cudaStream_t s);
 template <typename T>
 void launch_bounce_back(const Geometry& g, const ParticleView& pv, const T* f,
                         int pushed_layout, const int32_t* isnodes, LinkSlab ls,
-                        double* fHIp, double* torqp, cudaStream_t s);
+                        double* fHIp, double* torqp, bool prep, cudaStream_t s);
 template <typename T>
 void launch_bounce_scatter(const Geometry& g, const ParticleView& pv, T* f,
                            int pushed_layout, LinkSlab ls, cudaStream_t s,
@@ -410,7 +419,7 @@ struct BoxParticles {
 // for nb boxes of the array, on s and aux; the caller waits for ev_links
 // before the next particle step
 void launch_particle_step_multi(const BoxParticles* boxes, int nb, int max_npart,
-                                long long max_reset, cudaStream_t s, cudaStream_t aux,
+                                long long max_reset, bool prep, cudaStream_t s, cudaStream_t aux,
                                 cudaEvent_t ev_fork, cudaEvent_t ev_join, cudaEvent_t ev_links);
 // FORCING of many boxes into table slot `slot`, keeping each box's state
 // before the update in `backup`

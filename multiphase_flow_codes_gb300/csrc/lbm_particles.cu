@@ -110,6 +110,187 @@ constexpr int MAXNEAR = 2048;  // fluid nodes within rad + 1.5 of one centre
 // otherwise, so the outcome is always the FP64 one.
 constexpr float kDecide = 4e-3f;
 
+// 1 / x for x in [1/2, 3] (the link-fraction denominators of the bounce-back).
+// FP64: Newton-Raphson reciprocal iteration r <- r + r (1 - x r) from a
+// single-precision seed; each step squares the relative error, so two steps
+// take the seed's 2^-22 below the FP64 rounding.  On this GPU FP64 issues at
+// a small fraction of the FP32 rate, and the iteration is 4 FMAs.
+__device__ __forceinline__ double recip_link(double x) {
+  const float xf = __double2float_rn(x);
+  float r0;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(xf));
+  double r = (double)r0;
+  double e = fma(-x, r, 1.0);
+  r = fma(r, e, r);
+  e = fma(-x, r, 1.0);
+  return fma(r, e, r);
+}
+__device__ __forceinline__ float recip_link(float x) { return __frcp_rn(x); }
+__device__ __forceinline__ double fma_r(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ float fma_r(float a, float b, float c) { return fmaf(a, b, c); }
+
+// Offsets of lattice nodes from a particle's centre, per axis: the offset
+// d = pnt - c of the link point pnt = i + 1/2 from the image c of the centre
+// nearest to it depends on the node's coordinate i alone, so it is tabulated
+// once per block for the coordinates around the centre that links reach
+// (links outside the table compute it directly, the same value), in FP64
+// whatever the link arithmetic R (an FP32 centre near x = 256 is off by 1.5e-5).
+template <typename R>
+struct LeverTable {
+  R del[3][kBounceSpan];
+  int lo[3], reach;  // first tabulated coordinate per axis; ceil(rad) + 3
+
+  __device__ __forceinline__ void fill(int p, const Geometry& g, const ParticleView& pv) {
+    if (threadIdx.x < 3)
+      lo[threadIdx.x] = (int)floor((double)pv.ypglb[3 * p + threadIdx.x]) - (kBounceSpan / 2);
+    // the link nodes lie within rad + sqrt(2) of the centre: the entries
+    // kBounceSpan / 2 +- (ceil(rad) + 3) of the table cover them
+    if (threadIdx.x == 0) reach = min((int)ceil(pv.rad) + 3, kBounceSpan / 2 - 1);
+    __syncthreads();
+    const int dlo = kBounceSpan / 2 - reach, span = 2 * reach + 1;
+    for (int t = threadIdx.x; t < 3 * span; t += blockDim.x) {
+      const int a = t / span, d = dlo + (t - a * span);
+      const bool periodic = !(g.channel && a == 0);
+      const double cen = pv.ypglb[3 * p + a];
+      const int n = a == 0 ? g.nx : (a == 1 ? g.ny : g.nz);
+      const int nh = a == 0 ? g.nxh : (a == 1 ? g.nyh : g.nzh);
+      int i = lo[a] + d;
+      if (periodic) i = ((i % n) + n) % n;
+      const double pnt = (double)(i + 1) - 0.5;
+      del[a][d] = R(pnt - (periodic ? near_img(cen, pnt, n, nh) : cen));
+    }
+    __syncthreads();
+  }
+  __device__ __forceinline__ R at(int a, int i, int n, int nhalf, bool periodic, int p,
+                                  const ParticleView& pv) const {
+    int d = i - lo[a];
+    if (periodic) d = d < 0 ? d + n : (d >= n ? d - n : d);
+    if (d >= kBounceSpan / 2 - reach && d <= kBounceSpan / 2 + reach) return del[a][d];
+    const double cen = pv.ypglb[3 * p + a];
+    const double pnt = (double)(i + 1) - 0.5;
+    return R(pnt - (periodic ? near_img(cen, pnt, n, nhalf) : cen));
+  }
+  // The reference's lever arm is r = d + alpha c (the boundary point); every
+  // quantity it enters is a product with c: the wall velocity
+  // c . (w + omega x r) = c . w + omega . (r x c) and the torque dff (r x c),
+  // and r x c = d x c.  So the per-link arithmetic needs only e = d x c, which
+  // for c in {-1, 0, 1}^3 is selects and one add.
+  __device__ __forceinline__ void lever(int i, int j, int k, int ix, int iy, int iz, const Geometry& g,
+                                        int p, const ParticleView& pv, R& ex, R& ey, R& ez) const {
+    const R dx = at(0, i, g.nx, g.nxh, !g.channel, p, pv);
+    const R dy = at(1, j, g.ny, g.nyh, true, p, pv);
+    const R dz = at(2, k, g.nz, g.nzh, true, p, pv);
+    // cb db - cc dc for cb, cc in {-1, 0, 1}: one add at most
+    auto cross = [](int cb, R db, int cc, R dc) -> R {
+      const R u = cb == 0 ? R(0) : flip_if(cb < 0, db);
+      if (cc == 0) return u;
+      const R v = flip_if(cc < 0, dc);
+      return cb == 0 ? flip_if(true, v) : u - v;
+    };
+    ex = cross(iz, dy, iy, dz);
+    ey = cross(ix, dz, iz, dx);
+    ez = cross(iy, dx, ix, dy);
+  }
+};
+
+// The five interpolation cases of beads_collision (B/partlib.f90:1439-1536)
+// as f9 = c1 ff1 + c2 ff2 + c3 ff3 - 6 w c4 (c . u_w), with the same
+// populations read and one division (for alpha > 1/2) shared by its two
+// cases, so that a warp with mixed cases evaluates one formula:
+//   alpha <= 1/2: ff2, ff3 = f(q) at x - c, x - 2c;  c4 = 1
+//     x - c solid (s1):  c1 = 1
+//     x - 2c solid (s2): c1 = 2 alpha, c2 = 1 - 2 alpha
+//     else:              c1 = alpha (1 + 2 alpha), c2 = 1 - 4 alpha^2,
+//                        c3 = -alpha (1 - 2 alpha)
+//   alpha > 1/2: ff2, ff3 = f(qbar) at x, x - c;  c4 = c1
+//     x - c solid:  c1 = 1 / (2 alpha), c2 = 1 - c1
+//     else:         c1 = 1 / (alpha (2 alpha + 1)),
+//                   c2 = (2 alpha - 1)(2 alpha + 1) c1, c3 = 1 - c1 - c2
+template <typename R>
+struct BounceCoef { R c1, c2, c3, c4; };
+// alpha <= 1/2 on the bit patterns (an integer compare; the same outcome
+// for every alpha but a NaN with the sign bit set)
+__device__ __forceinline__ bool alpha_low(double a) {
+  return __double_as_longlong(a) <= __double_as_longlong(0.5);
+}
+__device__ __forceinline__ bool alpha_low(float a) { return __float_as_int(a) <= __float_as_int(0.5f); }
+template <typename R>
+__device__ __forceinline__ BounceCoef<R> bounce_coef(R alpha, bool low, bool s1, bool s2) {
+  const R t2 = alpha + alpha;
+  const R opt = R(1.0) + t2;             // 1 + 2 alpha
+  const R omt = R(1.0) - t2;             // 1 - 2 alpha
+  const R xa = alpha * opt;              // alpha (1 + 2 alpha)
+  const R y4 = omt * opt;                // 1 - 4 alpha^2
+  const R rc = recip_link(low ? R(1.0) : (s1 ? alpha : xa));
+  BounceCoef<R> c;
+  if (low) {
+    c.c1 = s1 ? R(1.0) : (s2 ? t2 : xa);
+    c.c2 = s1 ? R(0.0) : (s2 ? omt : y4);
+    c.c3 = (s1 || s2) ? R(0.0) : -alpha * omt;
+    c.c4 = R(1.0);
+  } else {
+    c.c1 = s1 ? R(0.5) * rc : rc;
+    c.c2 = s1 ? R(1.0) - c.c1 : -y4 * rc;
+    c.c3 = s1 ? R(0.0) : R(1.0) - c.c1 - c.c2;
+    c.c4 = c.c1;
+  }
+  return c;
+}
+
+// element of the populations' buffer that holds post-collision population q
+// of node (i, j, k) (0-based) in either layout (19 N < 2^31: N < 2^26 is
+// enforced).  pushed: the fused kernel has already moved it to its streaming
+// target (or bounced it back in place at a channel wall).
+__device__ __forceinline__ int post_index(const Geometry& g, bool pushed, int q, int i, int j, int k) {
+  const int N = (int)g.N;
+  if (!pushed) return q * N + i + g.nx * (j + g.ny * k);
+  const int it = i + cix(q);
+  if (g.channel && (it < 0 || it >= g.nx)) return ipopp(q) * N + i + g.nx * (j + g.ny * k);
+  return q * N + wrapi(it, g.nx) + g.nx * (wrapi(j + ciy(q), g.ny) + g.ny * wrapi(k + ciz(q), g.nz));
+}
+
+// What the bounce-back reads and weighs for one link: the elements that ff1,
+// ff2 and ff3 are (-1: none) and the coefficients.
+template <typename R>
+struct LinkPlan {
+  int g1, g2, g3;
+  BounceCoef<R> c;
+};
+template <typename R>
+__device__ __forceinline__ LinkPlan<R> plan_link(const Geometry& g, const uint32_t* mask, bool pushed, int ipop,
+                                                  int i, int j, int k, R alpha) {
+  const int ipp = ipopp(ipop);
+  const int ix = cix(ipop), iy = ciy(ipop), iz = ciz(ipop);
+  int im1 = i - ix, im2 = i - 2 * ix;
+  const int jm1 = wrapi(j - iy, g.ny), km1 = wrapi(k - iz, g.nz);
+  const int jm2 = wrapi(j - 2 * iy, g.ny), km2 = wrapi(k - 2 * iz, g.nz);
+  bool out1 = false, out2 = false;
+  if (g.channel) {
+    out1 = im1 < 0 || im1 >= g.nx;
+    out2 = im2 < 0 || im2 >= g.nx;
+  } else {
+    im1 = wrapi(im1, g.nx);
+    im2 = wrapi(im2, g.nx);
+  }
+  const bool low = alpha_low(alpha);
+  // (a point beyond a channel wall counts as solid)
+  const bool sol1 = out1 || is_solid(mask, g, km1 * g.ny + jm1, im1);
+  const bool sol2 = low && (out2 || is_solid(mask, g, km2 * g.ny + jm2, im2));
+  const bool s1 = sol1, s2 = sol2 && !s1;
+  LinkPlan<R> o;
+  o.g1 = post_index(g, pushed, ipop, i, j, k);
+  o.g2 = o.g3 = -1;
+  if (low) {
+    if (!s1) o.g2 = post_index(g, pushed, ipop, im1, jm1, km1);
+    if (!s1 && !s2) o.g3 = post_index(g, pushed, ipop, im2, jm2, km2);
+  } else {
+    o.g2 = post_index(g, pushed, ipp, i, j, k);
+    if (!s1) o.g3 = post_index(g, pushed, ipp, im1, jm1, km1);
+  }
+  o.c = bounce_coef<R>(alpha, low, s1, s2);
+  return o;
+}
+
 // beads_links for one particle per block.  Integer outcomes (solid flags,
 // link sets) are exactly those of the reference's FP64 loop nest; the link
 // fraction alpha is computed in FP64 (alpha_fp32 0: stored FP64; 2: stored
@@ -391,9 +572,12 @@ __global__ void __launch_bounds__(PB) k_flags(Geometry g, ParticleView pv, int32
 // The boundary links of one particle per block and what the bounce-back
 // needs of each: the next bounce-back is their first reader, so this runs
 // beside the refill and the next stream + collide.
+template <bool PREP>
 __device__ __forceinline__ void k_links_body(int p, const Geometry& g, const ParticleView& pv,
-                                              const LinkSlab& ls, DevStatus* st, int alpha_fp32) {
+                                              const int32_t* __restrict__ isnodes, const LinkSlab& ls,
+                                              DevStatus* st, int alpha_fp32) {
   __shared__ LinkSetup S;
+  __shared__ typename std::conditional<PREP, LeverTable<float>, int>::type levers;
   __shared__ int base;
   __shared__ int near_rc[MAXNEAR];  // fluid nodes within reach: row << 8 | candidate
   __shared__ int nnear;
@@ -408,6 +592,7 @@ __device__ __forceinline__ void k_links_body(int p, const Geometry& g, const Par
     }
     return;
   }
+  if constexpr (PREP) levers.fill(p, g, pv);
   const double rad2 = S.par[1];
   const float rad2f = S.parf[0], reachf = S.parf[1];
   const Cands& cx = S.cands[1];
@@ -550,7 +735,25 @@ __device__ __forceinline__ void k_links_body(int p, const Geometry& g, const Par
         const float a0 = diag ? 0.5f * bb : bb;
         const float ca = diag ? 0.5f * cc : cc;
         const float a1 = sqrtf(fmaxf(a0 * a0 - ca, 0.0f));
-        alph32[w] = 1.0f - (-a0 + a1);
+        const float alpha = 1.0f - (-a0 + a1);
+        alph32[w] = alpha;
+        if constexpr (PREP) {
+          const int ni = li - 1, nj = S.row_j[lr] - 1, nk = S.row_k[lr] - 1;
+          const LinkPlan<float> pl = plan_link<float>(g, solid_mask(isnodes, g), true, ipop, ni, nj, nk, alpha);
+          float ex, ey, ez;
+          levers.lever(ni, nj, nk, ix, iy, iz, g, p, pv, ex, ey, ez);
+          int32_t* gt = ls.gather + 3LL * p * ls.cap + w;
+          float* cf = ls.coef + 6LL * p * ls.cap + w;
+          gt[0] = pl.g1 | (alpha_low(alpha) ? 0 : (int)0x80000000);
+          gt[ls.cap] = pl.g2;
+          gt[2 * ls.cap] = pl.g3;
+          cf[0] = pl.c.c1;
+          cf[ls.cap] = pl.c.c2;
+          cf[2 * ls.cap] = pl.c.c3;
+          cf[3 * ls.cap] = ex;
+          cf[4 * ls.cap] = ey;
+          cf[5 * ls.cap] = ez;
+        }
       } else {
         // the components of c are +-1 or 0: c . x1 is selects and one add
         auto pick = [](int c, double v) { return flip_if(c < 0, v); };
@@ -585,9 +788,10 @@ __device__ __forceinline__ void k_links_body(int p, const Geometry& g, const Par
     if (!S.fixed_ok) raise_error(st, LBM_ERR_STATE, p);
   }
 }
-__global__ void __launch_bounds__(PB) k_links(Geometry g, ParticleView pv, LinkSlab ls, DevStatus* st,
-                                              int alpha_fp32) {
-  k_links_body(blockIdx.x, g, pv, ls, st, alpha_fp32);
+template <bool PREP>
+__global__ void __launch_bounds__(PB) k_links(Geometry g, ParticleView pv, const int32_t* isnodes,
+                                              LinkSlab ls, DevStatus* st, int alpha_fp32) {
+  k_links_body<PREP>(blockIdx.x, g, pv, isnodes, ls, st, alpha_fp32);
 }
 
 // running sum: plain FP64, or FP32 with Kahan compensation (FP32 path)
@@ -610,25 +814,6 @@ struct Acc<float> {
   __device__ void add_prod(float a, float b) { add(a * b); }
   __device__ double value() const { return (double)s - (double)c; }
 };
-
-// 1 / x for x in [1/2, 3] (the link-fraction denominators of the bounce-back).
-// FP64: Newton-Raphson reciprocal iteration r <- r + r (1 - x r) from a
-// single-precision seed; each step squares the relative error, so two steps
-// take the seed's 2^-22 below the FP64 rounding.  On this GPU FP64 issues at
-// a small fraction of the FP32 rate, and the iteration is 4 FMAs.
-__device__ __forceinline__ double recip_link(double x) {
-  const float xf = __double2float_rn(x);
-  float r0;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(xf));
-  double r = (double)r0;
-  double e = fma(-x, r, 1.0);
-  r = fma(r, e, r);
-  e = fma(-x, r, 1.0);
-  return fma(r, e, r);
-}
-__device__ __forceinline__ float recip_link(float x) { return __frcp_rn(x); }
-__device__ __forceinline__ double fma_r(double a, double b, double c) { return fma(a, b, c); }
-__device__ __forceinline__ float fma_r(float a, float b, float c) { return fmaf(a, b, c); }
 
 // a stored population: FP64 populations are 64-bit fixed point while
 // g.pop_fixed is set (between fused steps of the FP64 plain path)
@@ -653,23 +838,6 @@ __device__ __forceinline__ void st_pop(const Geometry& g, T* f, long long idx, T
   f[idx] = v;
 }
 
-// post-collision population q at node (i, j, k) (0-based) in either layout.
-// pushed: the fused kernel has already moved it to its streaming target
-// (or bounced it back in place at a channel wall).
-template <typename T>
-__device__ __forceinline__ T read_post(const Geometry& g, const T* f, int pushed, int q, int i,
-                                       int j, int k) {
-  // 32-bit element indices: 19 N < 2^31 (N < 2^26 is enforced)
-  const int N = (int)g.N;
-  const int n = i + g.nx * (j + g.ny * k);
-  if (!pushed) return ld_pop(g, f, q * N + n);
-  int it = i + cix(q);
-  if (g.channel && (it < 0 || it >= g.nx)) return ld_pop(g, f, ipopp(q) * N + n);
-  it = wrapi(it, g.nx);
-  const int jt = wrapi(j + ciy(q), g.ny), kt = wrapi(k + ciz(q), g.nz);
-  return ld_pop(g, f, q * N + it + g.nx * (jt + g.ny * kt));
-}
-
 // threads per block of the bounce-back: small blocks leave fewer idle lanes in
 // the last pass over a particle's ~1000 links (1000 spheres at 256^3, FP32:
 // 256 threads 75 us, 128 threads 72 us); FP64, two blocks of 64 threads a
@@ -688,183 +856,84 @@ constexpr int bounce_blocks() { return 1024 / bounce_threads<T>(); }  // residen
 // the GPU idle for some ten passes: 64^3 with 16 spheres took 84 us, split in
 // eleven 17 us.  The block that finishes last adds the partial sums in block
 // order.
-template <typename T, int NT>
-__device__ __forceinline__ void k_bounce_body(int bx, int split, Geometry g, ParticleView pv, const T* f, int pushed,
-                                               const int32_t* __restrict__ isnodes, LinkSlab ls,
+// PREP (FP32, pushed populations): the gathers, coefficients and lever arms
+// of the links come from the link build, which runs beside the previous refill
+// and the stream + collide; a pass is then one round of coalesced loads and
+// one of gathers (32^3 with 5 spheres: 47 -> 21 us a step, 160^3 with 300:
+// 50 -> 36).  With many spheres forming them there costs the build more than
+// it saves here (256^3 with 1000: 0.61 -> 0.66 ms a step), so kPrepParticles
+// limits it.
+template <typename T, int NT, bool PREP>
+__device__ __forceinline__ void k_bounce_body(int bx, int split, const Geometry& g, const ParticleView& pv,
+                                               const T* __restrict__ f, int pushed,
+                                               const int32_t* __restrict__ isnodes, const LinkSlab& ls,
                                                double* fHIp, double* torqp) {
   const int p = bx / split, part_id = bx - p * split;
   if (p >= pv.npart) return;
   const int cnt = ls.count[p];
-  const int32_t* code = ls.code + (long long)p * ls.cap;
+  const int32_t* __restrict__ code = ls.code + (long long)p * ls.cap;
   // link fractions and bounced populations are stored in the population
   // precision (FP32 slabs reuse the first half of the FP64 arrays)
-  const T* alph = reinterpret_cast<const T*>(ls.alpha + (long long)p * ls.cap);
+  const T* __restrict__ alph = reinterpret_cast<const T*>(ls.alpha + (long long)p * ls.cap);
   T* f9s = reinterpret_cast<T*>(ls.f9 + (long long)p * ls.cap);
+  const int32_t* __restrict__ gather = PREP ? ls.gather + 3LL * p * ls.cap : nullptr;
+  const float* __restrict__ coef = PREP ? ls.coef + 6LL * p * ls.cap : nullptr;
   // per-link arithmetic in the population precision R (FP64 plain path,
   // FP32 shifted path)
   using R = T;
   Acc<T> acc6[6];
-  // the particle's velocities in the arithmetic precision and the first
-  // tabulated coordinate per axis, formed once by thread 0 (conversions and
-  // roundings of FP64 values issue on the FP64 pipe, and cost a warp the same
-  // whatever its active lanes)
+  // the particle's velocities in the arithmetic precision, formed once
+  // (conversions and roundings of FP64 values issue on the FP64 pipe, and
+  // cost a warp the same whatever its active lanes)
   __shared__ R s_wo[6];
-  __shared__ int s_lo[4];
-  if (threadIdx.x == 0) {
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      s_wo[a] = R(pv.wp[3 * p + a]);
-      s_wo[3 + a] = R(pv.omgp[3 * p + a]);
-      s_lo[a] = (int)floor((double)pv.ypglb[3 * p + a]) - (kBounceSpan / 2);
-    }
-    // the link nodes lie within rad + sqrt(2) of the centre: the entries
-    // kBounceSpan / 2 +- (ceil(rad) + 3) of the table cover them
-    s_lo[3] = min((int)ceil(pv.rad) + 3, kBounceSpan / 2 - 1);
+  __shared__ R tcw[NPOP];  // c_q . w
+  if (threadIdx.x < 6)
+    s_wo[threadIdx.x] = R(threadIdx.x < 3 ? pv.wp[3 * p + threadIdx.x] : pv.omgp[3 * p + threadIdx.x - 3]);
+  __shared__ typename std::conditional<PREP, int, LeverTable<R>>::type levers;
+  if constexpr (!PREP) levers.fill(p, g, pv);
+  else __syncthreads();
+  if (threadIdx.x < NPOP) {
+    // c_a v with c_a in {-1, 0, 1}: exact, so selected rather than multiplied
+    auto sel = [](int c, R v) { return c == 0 ? R(0) : flip_if(c < 0, v); };
+    const int q = threadIdx.x;
+    tcw[q] = sel(cix(q), s_wo[0]) + sel(ciy(q), s_wo[1]) + sel(ciz(q), s_wo[2]);
   }
   __syncthreads();
-  const R w1 = s_wo[0], w2 = s_wo[1], w3 = s_wo[2];
   const R omg1 = s_wo[3], omg2 = s_wo[4], omg3 = s_wo[5];
-  const R xc0 = R(0), yc0 = R(0), zc0 = R(0);  // (unused by delta)
-  const bool channel = g.channel != 0;
-  const uint32_t* mask = solid_mask(isnodes, g);
-  // Per axis, the offset d = pnt - c of the link point pnt = i + 1/2 from the
-  // image c of the centre nearest to it depends on the node's coordinate i
-  // alone: tabulate it once per particle for the coordinates around the
-  // centre that links reach (same operations as per link, so the same
-  // values); links outside the table compute it directly.  Per direction,
-  // c_q . w.
-  __shared__ R tdel[3][kBounceSpan];
-  __shared__ R tcw[NPOP];
-  // c_a v with c_a in {-1, 0, 1}: exact, so selected rather than multiplied
-  auto sel = [](int c, R v) { return c == 0 ? R(0) : flip_if(c < 0, v); };
-  const int lo[3] = {s_lo[0], s_lo[1], s_lo[2]};
-  const int dlo = kBounceSpan / 2 - s_lo[3], dhi = kBounceSpan / 2 + s_lo[3];
-  {
-    // selects rather than arrays indexed by a, which would live in local memory
-    const int span = dhi - dlo + 1;
-    for (int t = threadIdx.x; t < 3 * span; t += NT) {
-      const int a = t / span, d = dlo + (t - a * span);
-      const bool periodic = !(channel && a == 0);
-      // in FP64 whatever R: an FP32 centre near x = 256 is off by 1.5e-5
-      const double cen = pv.ypglb[3 * p + a];
-      const int n = a == 0 ? g.nx : (a == 1 ? g.ny : g.nz);
-      const int nh = a == 0 ? g.nxh : (a == 1 ? g.nyh : g.nzh);
-      int i = (a == 0 ? lo[0] : (a == 1 ? lo[1] : lo[2])) + d;
-      if (periodic) i = ((i % n) + n) % n;
-      const double pnt = (double)(i + 1) - 0.5;
-      tdel[a][d] = R(pnt - (periodic ? near_img_t<double>(cen, pnt, n, nh) : cen));
-    }
-    if (threadIdx.x < NPOP) {
-      const int q = threadIdx.x;
-      tcw[q] = sel(cix(q), w1) + sel(ciy(q), w2) + sel(ciz(q), w3);
-    }
-    __syncthreads();
-  }
-  auto delta = [&](int a, int i, R, int n, int nhalf, bool periodic) -> R {
-    int d = i - lo[a];
-    if (periodic) d = d < 0 ? d + n : (d >= n ? d - n : d);
-    if (d >= dlo && d <= dhi) return tdel[a][d];
-    const double cen = pv.ypglb[3 * p + a];
-    const double pnt = (double)(i + 1) - 0.5;
-    return R(pnt - (periodic ? near_img_t<double>(cen, pnt, n, nhalf) : cen));
-  };
-  // cb db - cc dc for cb, cc in {-1, 0, 1}: one add at most
-  auto cross = [](int cb, R db, int cc, R dc) -> R {
-    const R u = cb == 0 ? R(0) : flip_if(cb < 0, db);
-    if (cc == 0) return u;
-    const R v = flip_if(cc < 0, dc);
-    return cb == 0 ? flip_if(true, v) : u - v;
-  };
-  // The reference's lever arm is r = d + alpha c (the boundary point);
-  // every quantity it enters is a product with c: the wall velocity
-  // c . (w + omega x r) = c . w + omega . (r x c) and the torque
-  // dff (r x c), and r x c = d x c.  So the per-link arithmetic needs only
-  // e = d x c, which for c in {-1, 0, 1}^3 is selects and one add.
-  auto lever = [&](int i, int j, int k, int ix, int iy, int iz, R& ex, R& ey, R& ez) {
-    const R dx = delta(0, i, xc0, g.nx, g.nxh, !channel);
-    const R dy = delta(1, j, yc0, g.ny, g.nyh, true);
-    const R dz = delta(2, k, zc0, g.nz, g.nzh, true);
-    ex = cross(iz, dy, iy, dz);
-    ey = cross(ix, dz, iz, dx);
-    ez = cross(iy, dx, ix, dy);
-  };
+  const uint32_t* mask = PREP ? nullptr : solid_mask(isnodes, g);
   for (int l = part_id * NT + threadIdx.x; l < cnt; l += split * NT) {
     // 32-bit decode: node < 2^26
     const int cd = code[l];
     const int ipop = cd & 31;
-    const int node = cd >> 5;
-    const int r = node / g.nx;
-    const int i = node - r * g.nx;
-    const int k = r / g.ny, j = r - k * g.ny;
-    const R alpha = alph[l];
-    const int ipp = ipopp(ipop);
     const int ix = cix(ipop), iy = ciy(ipop), iz = ciz(ipop);
-    int im1 = i - ix, im2 = i - 2 * ix;
-    const int jm1 = wrapi(j - iy, g.ny), km1 = wrapi(k - iz, g.nz);
-    const int jm2 = wrapi(j - 2 * iy, g.ny), km2 = wrapi(k - 2 * iz, g.nz);
-    bool out1 = false, out2 = false;
-    if (channel) {
-      out1 = im1 < 0 || im1 >= g.nx;
-      out2 = im2 < 0 || im2 >= g.nx;
-    } else {
-      im1 = wrapi(im1, g.nx);
-      im2 = wrapi(im2, g.nx);
-    }
+    LinkPlan<R> pl;
     R ex, ey, ez;
-    lever(i, j, k, ix, iy, iz, ex, ey, ez);
+    if constexpr (PREP) {
+      const int g1 = gather[l];
+      pl.g1 = g1 & 0x7fffffff;  // bit 31: alpha > 1/2
+      pl.g2 = gather[ls.cap + l];
+      pl.g3 = gather[2 * ls.cap + l];
+      pl.c.c1 = coef[l];
+      pl.c.c2 = coef[ls.cap + l];
+      pl.c.c3 = coef[2 * ls.cap + l];
+      pl.c.c4 = g1 < 0 ? pl.c.c1 : R(1.0);
+      ex = coef[3 * ls.cap + l];
+      ey = coef[4 * ls.cap + l];
+      ez = coef[5 * ls.cap + l];
+    } else {
+      const int node = cd >> 5;
+      const int r = node / g.nx;
+      const int i = node - r * g.nx;
+      const int k = r / g.ny, j = r - k * g.ny;
+      levers.lever(i, j, k, ix, iy, iz, g, p, pv, ex, ey, ez);
+      pl = plan_link<R>(g, mask, pushed != 0, ipop, i, j, k, alph[l]);
+    }
     const R uwpro = fma_r(omg1, ex, fma_r(omg2, ey, fma_r(omg3, ez, tcw[ipop])));
-    const R ff1 = R(read_post(g, f, pushed, ipop, i, j, k));
-    // The five interpolation cases of beads_collision (B/partlib.f90:1439-1536)
-    // as f9 = c1 ff1 + c2 ff2 + c3 ff3 - 6 w c4 (c . u_w), with the same
-    // populations read and one division (for alpha > 1/2) shared by its two
-    // cases, so that a warp with mixed cases evaluates one formula:
-    //   alpha <= 1/2: ff2, ff3 = f(q) at x - c, x - 2c
-    //     x - c solid:  c1 = 1
-    //     x - 2c solid: c1 = 2 alpha, c2 = 1 - 2 alpha
-    //     else:         c1 = alpha (1 + 2 alpha), c2 = 1 - 4 alpha^2,
-    //                   c3 = -alpha (1 - 2 alpha)
-    //   alpha > 1/2: ff2, ff3 = f(qbar) at x, x - c;  c4 = c1
-    //     x - c solid:  c1 = 1 / (2 alpha), c2 = 1 - c1
-    //     else:         c1 = 1 / (alpha (2 alpha + 1)),
-    //                   c2 = (2 alpha - 1)(2 alpha + 1) c1, c3 = 1 - c1 - c2
-    // alpha <= 1/2 on the bit patterns (an integer compare; the same outcome
-    // for every alpha but a NaN with the sign bit set)
-    bool low;
-    if constexpr (sizeof(R) == 8) low = __double_as_longlong(alpha) <= __double_as_longlong(0.5);
-    else low = __float_as_int(alpha) <= __float_as_int(0.5f);
-    int ibm1 = 2, ibm2 = 2;
-    if (!out1) ibm1 = is_solid(mask, g, km1 * g.ny + jm1, im1) ? 1 : -1;
-    if (low && !out2) ibm2 = is_solid(mask, g, km2 * g.ny + jm2, im2) ? 1 : -1;
-    const bool s1 = ibm1 > 0;
-    const bool s2 = low && !s1 && ibm2 > 0;
-    R ff2 = R(0), ff3 = R(0);
-    if (low) {
-      if (!s1) ff2 = R(read_post(g, f, pushed, ipop, im1, jm1, km1));
-      if (!s1 && !s2) ff3 = R(read_post(g, f, pushed, ipop, im2, jm2, km2));
-    } else {
-      ff2 = R(read_post(g, f, pushed, ipp, i, j, k));
-      if (!s1) ff3 = R(read_post(g, f, pushed, ipp, im1, jm1, km1));
-    }
-    const R t2 = alpha + alpha;
-    const R opt = R(1.0) + t2;             // 1 + 2 alpha
-    const R omt = R(1.0) - t2;             // 1 - 2 alpha
-    const R xa = alpha * opt;              // alpha (1 + 2 alpha)
-    const R y4 = omt * opt;                // 1 - 4 alpha^2
-    const R rc = recip_link(low ? R(1.0) : (s1 ? alpha : xa));
-    R c1, c2, c3, c4;
-    if (low) {
-      c1 = s1 ? R(1.0) : (s2 ? t2 : xa);
-      c2 = s1 ? R(0.0) : (s2 ? omt : y4);
-      c3 = (s1 || s2) ? R(0.0) : -alpha * omt;
-      c4 = R(1.0);
-    } else {
-      c1 = s1 ? R(0.5) * rc : rc;
-      c2 = s1 ? R(1.0) - c1 : -y4 * rc;
-      c3 = s1 ? R(0.0) : R(1.0) - c1 - c2;
-      c4 = c1;
-    }
+    const R ff1 = R(ld_pop(g, f, (long long)pl.g1));
+    const R ff2 = pl.g2 >= 0 ? R(ld_pop(g, f, (long long)pl.g2)) : R(0);
+    const R ff3 = pl.g3 >= 0 ? R(ld_pop(g, f, (long long)pl.g3)) : R(0);
     const R k6 = ipop <= 6 ? R(6.0 / 18.0) : R(6.0 / 36.0);
-    const R f9 = fma_r(c1, ff1, fma_r(c2, ff2, fma_r(c3, ff3, -(k6 * c4) * uwpro)));
+    const R f9 = fma_r(pl.c.c1, ff1, fma_r(pl.c.c2, ff2, fma_r(pl.c.c3, ff3, -(k6 * pl.c.c4) * uwpro)));
     f9s[l] = f9;
     const R dff = ff1 + f9;
     if (ix) acc6[0].add(flip_if(ix < 0, dff));
@@ -942,13 +1011,13 @@ __device__ __forceinline__ void k_bounce_body(int bx, int split, Geometry g, Par
     }
   }
 }
-template <typename T>
+template <typename T, bool PREP>
 // (64 registers: 1024 threads per SM, so that the 1000 spheres of the
 // workload take one wave)
 __global__ void __launch_bounds__(bounce_threads<T>(), bounce_blocks<T>()) k_bounce(Geometry g, ParticleView pv, const T* f, int pushed,
                                                const int32_t* __restrict__ isnodes, LinkSlab ls,
                                                double* fHIp, double* torqp, int split) {
-  k_bounce_body<T, bounce_threads<T>()>(blockIdx.x, split, g, pv, f, pushed, isnodes, ls, fHIp, torqp);
+  k_bounce_body<T, bounce_threads<T>(), PREP>(blockIdx.x, split, g, pv, f, pushed, isnodes, ls, fHIp, torqp);
 }
 
 // the bounce-back stores of beads_collision: f(ipp, x + c) = f9
@@ -1497,17 +1566,19 @@ void launch_flags(const Geometry& g, const ParticleView& pv, int32_t* isnodes, L
   if (pv.npart <= 0) return;
   { k_flags<<<pv.npart, PB, 0, s>>>(g, pv, isnodes, ls); count_launch(); }
 }
-void launch_link_lists(const Geometry& g, const ParticleView& pv, LinkSlab ls, DevStatus* st,
-                       int alpha_fp32, cudaStream_t s) {
+void launch_link_lists(const Geometry& g, const ParticleView& pv, const int32_t* isnodes, LinkSlab ls,
+                       DevStatus* st, int alpha_fp32, bool prep, cudaStream_t s) {
   if (pv.npart <= 0) return;
-  { k_links<<<pv.npart, PB, 0, s>>>(g, pv, ls, st, alpha_fp32); count_launch(); }
+  if (prep) k_links<true><<<pv.npart, PB, 0, s>>>(g, pv, isnodes, ls, st, alpha_fp32);
+  else k_links<false><<<pv.npart, PB, 0, s>>>(g, pv, isnodes, ls, st, alpha_fp32);
+  count_launch();
 }
 void launch_links(const Geometry& g, const ParticleView& pv, int32_t* isnodes, LinkSlab ls,
-                  DevStatus* st, int alpha_fp32, cudaStream_t s) {
+                  DevStatus* st, int alpha_fp32, bool prep, cudaStream_t s) {
   if (pv.npart <= 0) return;
   { k_link_sweeps<<<(3 * pv.npart + kSmallBlock - 1) / kSmallBlock, kSmallBlock, 0, s>>>(g, pv, ls); count_launch(); }
   launch_flags(g, pv, isnodes, ls, s);
-  launch_link_lists(g, pv, ls, st, alpha_fp32, s);
+  launch_link_lists(g, pv, isnodes, ls, st, alpha_fp32, prep, s);
 }
 
 // Blocks that share a particle's bounce-back (FP64): as many as take one
@@ -1524,10 +1595,17 @@ int bounce_split(double rad, long long npart) {
 template <typename T>
 void launch_bounce_back(const Geometry& g, const ParticleView& pv, const T* f, int pushed,
                         const int32_t* isnodes, LinkSlab ls, double* fHIp, double* torqp,
-                        cudaStream_t s) {
+                        bool prep, cudaStream_t s) {
   if (pv.npart <= 0) return;
   const int split = bounce_split<T>(pv.rad, pv.npart);
-  { k_bounce<T><<<pv.npart * split, bounce_threads<T>(), 0, s>>>(g, pv, f, pushed, isnodes, ls, fHIp, torqp, split); count_launch(); }
+  count_launch();
+  if constexpr (sizeof(T) == 4) {
+    if (prep && pushed) {
+      k_bounce<T, true><<<pv.npart, bounce_threads<T>(), 0, s>>>(g, pv, f, pushed, isnodes, ls, fHIp, torqp, 1);
+      return;
+    }
+  }
+  k_bounce<T, false><<<pv.npart * split, bounce_threads<T>(), 0, s>>>(g, pv, f, pushed, isnodes, ls, fHIp, torqp, split);
 }
 
 template <typename T>
@@ -1599,10 +1677,11 @@ namespace {
   const int nblk = (nblocks_expr);                   \
   if ((int)blockIdx.x >= nblk) return;
 
+template <bool PREP>
 __global__ void __launch_bounds__(bounce_threads<float>(), bounce_blocks<float>()) k_bounce_multi(const BoxParticles* boxes) {
   BOX_OR_RETURN(B.pv.npart)
-  k_bounce_body<float, bounce_threads<float>()>(blockIdx.x, 1, B.g, B.pv, B.f, 1, B.flags_cur, B.ls,
-                                                B.ms.fHIp, B.ms.torqp);
+  k_bounce_body<float, bounce_threads<float>(), PREP>(blockIdx.x, 1, B.g, B.pv, B.f, 1, B.flags_cur, B.ls,
+                                                      B.ms.fHIp, B.ms.torqp);
 }
 __global__ void __launch_bounds__(PB) k_bounce_store_multi(const BoxParticles* boxes) {
   BOX_OR_RETURN(B.pv.npart)
@@ -1640,9 +1719,10 @@ __global__ void __launch_bounds__(PB) k_flags_multi(const BoxParticles* boxes) {
   BOX_OR_RETURN(B.pv.npart)
   k_flags_body(blockIdx.x, B.g, B.pv, B.flags_next, B.ls);
 }
+template <bool PREP>
 __global__ void __launch_bounds__(PB) k_links_multi(const BoxParticles* boxes) {
   BOX_OR_RETURN(B.pv.npart)
-  k_links_body(blockIdx.x, B.g, B.pv, B.ls, B.st, 1);
+  k_links_body<PREP>(blockIdx.x, B.g, B.pv, B.flags_next, B.ls, B.st, 1);
 }
 __global__ void __launch_bounds__(PB) k_fill_detect_multi(const BoxParticles* boxes) {
   BOX_OR_RETURN(B.pv.npart)
@@ -1665,7 +1745,7 @@ __global__ void __launch_bounds__(128) k_fill_events_multi(const BoxParticles* b
 // overlap check beside move and flags, the link lists (ev_links) beside the
 // refill and the next stream + collide.
 void launch_particle_step_multi(const BoxParticles* boxes, int nb, int max_npart,
-                                long long max_reset, cudaStream_t s, cudaStream_t aux,
+                                long long max_reset, bool prep, cudaStream_t s, cudaStream_t aux,
                                 cudaEvent_t ev_fork, cudaEvent_t ev_join, cudaEvent_t ev_links) {
   if (nb <= 0 || max_npart <= 0) return;
   auto grid = [&](long long blocks) { return dim3((unsigned)(blocks > 0 ? blocks : 1), nb); };
@@ -1681,7 +1761,9 @@ void launch_particle_step_multi(const BoxParticles* boxes, int nb, int max_npart
   const long long rb = (max_reset + 256 * 8 - 1) / (256 * 8);
   k_reset_multi<<<grid(rb < 1024 ? rb : 1024), 256, 0, aux>>>(boxes); count_launch();
   k_lubforce_multi<<<grid((max_npart * 32 + 127) / 128), 128, 0, aux>>>(boxes); count_launch();
-  k_bounce_multi<<<grid(max_npart), bounce_threads<float>(), 0, s>>>(boxes); count_launch();
+  if (prep) k_bounce_multi<true><<<grid(max_npart), bounce_threads<float>(), 0, s>>>(boxes);
+  else k_bounce_multi<false><<<grid(max_npart), bounce_threads<float>(), 0, s>>>(boxes);
+  count_launch();
   join();
   fork();
   k_bounce_store_multi<<<grid(max_npart), PB, 0, aux>>>(boxes); count_launch();
@@ -1691,7 +1773,9 @@ void launch_particle_step_multi(const BoxParticles* boxes, int nb, int max_npart
   k_flags_multi<<<grid(max_npart), PB, 0, s>>>(boxes); count_launch();
   join();
   fork();
-  k_links_multi<<<grid(max_npart), PB, 0, aux>>>(boxes); count_launch();
+  if (prep) k_links_multi<true><<<grid(max_npart), PB, 0, aux>>>(boxes);
+  else k_links_multi<false><<<grid(max_npart), PB, 0, aux>>>(boxes);
+  count_launch();
   cudaEventRecord(ev_links, aux);
   k_fill_detect_multi<<<grid(max_npart), PB, 0, s>>>(boxes); count_launch();
   k_fill_events_multi<<<grid(kFillBlocks), 128, 0, s>>>(boxes); count_launch();
@@ -1699,9 +1783,9 @@ void launch_particle_step_multi(const BoxParticles* boxes, int nb, int max_npart
 
 template void launch_bounce_back<double>(const Geometry&, const ParticleView&, const double*,
                                          int, const int32_t*, LinkSlab, double*, double*,
-                                         cudaStream_t);
+                                         bool, cudaStream_t);
 template void launch_bounce_back<float>(const Geometry&, const ParticleView&, const float*, int,
-                                        const int32_t*, LinkSlab, double*, double*,
+                                        const int32_t*, LinkSlab, double*, double*, bool,
                                         cudaStream_t);
 template void launch_bounce_scatter<double>(const Geometry&, const ParticleView&, double*, int,
                                             LinkSlab, cudaStream_t, DevStatus*);
