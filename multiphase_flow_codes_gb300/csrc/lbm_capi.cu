@@ -947,6 +947,7 @@ int lbm_create(const lbm_config* cfg, lbm_ctx** out) {
   Geometry& g = ctx->g;
   g.nx = cfg->nx; g.ny = cfg->ny; g.nz = cfg->nz;
   g.nxh = g.nx / 2; g.nyh = g.ny / 2; g.nzh = g.nz / 2;
+  g.inv_nx = div_inv(g.nx); g.inv_ny = div_inv(g.ny);
   g.N = (long long)g.nx * g.ny * g.nz;
   g.channel = cfg->boundary == LBM_BC_XWALLS;
   g.sw = 4 * ((g.nx + 127) / 128);
@@ -1320,6 +1321,7 @@ int lbm_place_particles(const lbm_config* cfg, int npart, int seed, int max_roun
   Geometry g{};
   g.nx = cfg->nx; g.ny = cfg->ny; g.nz = cfg->nz;
   g.nxh = g.nx / 2; g.nyh = g.ny / 2; g.nzh = g.nz / 2;
+  g.inv_nx = div_inv(g.nx); g.inv_ny = div_inv(g.ny);
   g.channel = cfg->boundary == LBM_BC_XWALLS;
   if (npart > 0 &&
       !init_particle_positions(g, npart, cfg->rad, cfg->mingap, cfg->mingap_w, seed,

@@ -220,11 +220,9 @@ __global__ void __launch_bounds__(128, FX ? 4 : 1) k_fused(Geometry g, RatesT<T>
                                                const int32_t* __restrict__ isnodes,
                                                ForceView<T> fprev, ForceView<T> fnew,
                                                T* fcache, int fcache_mode) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  const int y = blockIdx.y, z = blockIdx.z;
-  if (x >= g.nx) return;
+  int n, x, y, z;
+  if (!node_at(g, n, x, y, z)) return;
   const int nx = g.nx, nxy = g.nx * g.ny, N = (int)g.N;
-  const int n = x + nx * y + nxy * z;
   T f[NPOP];
   T fp[3];
   // the cached force is loaded with the populations (same latency)
@@ -355,7 +353,7 @@ __device__ __forceinline__ void body_force_fxd(const ForceView<double>& fv, cons
 // (256^3 with 1000 spheres: 1.01 ms, 5.0 TB/s of populations; four CTAs at
 // 128 registers 1.11 ms, three 1.24 ms, six 1.02 ms; before, with 128-bit
 // products, 1.54 ms at four).
-template <bool CHANNEL, bool INTCORE>
+template <bool CHANNEL, bool INTCORE, bool ROWS>
 __global__ void __launch_bounds__(128, 5) k_fused_fixed(Geometry g, RatesT<double> r,
                                                          const long long* __restrict__ fin,
                                                          long long* __restrict__ fout,
@@ -364,11 +362,9 @@ __global__ void __launch_bounds__(128, 5) k_fused_fixed(Geometry g, RatesT<doubl
                                                          ForceView<double> fnew,
                                                          long long* fcache, int fcache_mode,
                                                          DevStatus* st) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  const int y = blockIdx.y, z = blockIdx.z;
-  if (x >= g.nx) return;
+  int n, x, y, z;
+  if (!node_at<ROWS>(g, n, x, y, z)) return;
   const int nx = g.nx, nxy = g.nx * g.ny, N = (int)g.N;
-  const int n = x + nx * y + nxy * z;
   long long f[NPOP];
   long long fp[3], fc[3];
   if (fcache_mode == 2) {
@@ -445,11 +441,9 @@ __global__ void k_pop_from_fixed(double* f, long long n) {
 // streaming alone (per-subroutine entry), B/streaming.f90:2-171
 template <typename T, bool CHANNEL>
 __global__ void k_stream(Geometry g, const T* __restrict__ fin, T* __restrict__ fout) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  const int y = blockIdx.y, z = blockIdx.z;
-  if (x >= g.nx) return;
+  int n, x, y, z;
+  if (!node_at(g, n, x, y, z)) return;
   const long long N = g.N;
-  const long long n = x + (long long)g.nx * (y + (long long)g.ny * z);
   fout[n] = fin[n];
 #pragma unroll
   for (int q = 1; q < NPOP; ++q) {
@@ -475,11 +469,9 @@ __global__ void __launch_bounds__(128, FX ? 4 : 1) k_collision(Geometry g, Rates
                             const int32_t* __restrict__ isnodes, ForceView<T> fv,
                             const T* __restrict__ rho, const T* __restrict__ ux,
                             const T* __restrict__ uy, const T* __restrict__ uz) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  const int y = blockIdx.y, z = blockIdx.z;
-  if (x >= g.nx) return;
+  int n, x, y, z;
+  if (!node_at(g, n, x, y, z)) return;
   const long long N = g.N;
-  const long long n = x + (long long)g.nx * (y + (long long)g.ny * z);
   if (isnodes[n] >= 0) return;
   T fl[NPOP];
 #pragma unroll
@@ -511,7 +503,7 @@ __global__ void __launch_bounds__(128, FX ? 4 : 1) k_collision(Geometry g, Rates
 // first: the collision uses the stored density (no iteration made these
 // populations).  before: the change the previous pass found; when it is within
 // eps or not finite the loop has ended, and this pass does nothing.
-template <bool CHANNEL>
+template <bool CHANNEL, bool ROWS>
 __global__ void __launch_bounds__(128, 4) k_relax(Geometry g, Rates r, RatesT<double> rt, const double* __restrict__ fin,
                             double* __restrict__ fout, const int32_t* __restrict__ isnodes,
                             ForceView<double> fv, double* __restrict__ rho,
@@ -523,12 +515,11 @@ __global__ void __launch_bounds__(128, 4) k_relax(Geometry g, Rates r, RatesT<do
     const double e = __longlong_as_double((long long)*before);
     if (e <= eps || isinf(e)) return;
   }
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  const int y = blockIdx.y, z = blockIdx.z;
+  int n, x, y, z;
+  const bool in = node_at<ROWS>(g, n, x, y, z);
   const int nx = g.nx, nxy = g.nx * g.ny, N = (int)g.N;
-  const int n = x + nx * y + nxy * z;
   double d = 0.0;
-  if (x < nx) {
+  if (in) {
     double f[NPOP];
 #pragma unroll
     for (int q = 0; q < NPOP; ++q) f[q] = fin[(size_t)q * N + n];
@@ -594,11 +585,9 @@ __global__ void k_macrovar(Geometry g, const T* __restrict__ f,
                            const int32_t* __restrict__ isnodes, ForceView<T> fv,
                            ParticleView pv, T* __restrict__ rho, T* __restrict__ ux,
                            T* __restrict__ uy, T* __restrict__ uz) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  const int y = blockIdx.y, z = blockIdx.z;
-  if (x >= g.nx) return;
+  int n, x, y, z;
+  if (!node_at(g, n, x, y, z)) return;
   const long long N = g.N;
-  const long long n = x + (long long)g.nx * (y + (long long)g.ny * z);
   T fl[NPOP];
 #pragma unroll
   for (int q = 0; q < NPOP; ++q) fl[q] = f[q * N + n];
@@ -824,10 +813,8 @@ __global__ void k_convert_back(const T* __restrict__ in, double* __restrict__ ou
 
 template <typename T>
 __global__ void k_force_field(Geometry g, ForceView<T> fv, double* fx, double* fy, double* fz) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  const int y = blockIdx.y, z = blockIdx.z;
-  if (x >= g.nx) return;
-  long long n = x + (long long)g.nx * (y + (long long)g.ny * z);
+  int n, x, y, z;
+  if (!node_at(g, n, x, y, z)) return;
   T a, b, c;
   body_force(fv, g, x, y, z, a, b, c);
   fx[n] = (double)a; fy[n] = (double)b; fz[n] = (double)c;
@@ -951,8 +938,13 @@ __global__ void k_force_rowtab(Geometry g, const T* __restrict__ ztab,
   k_force_rowtab_body<T>(blockIdx.x, gridDim.x, g, ztab, ytw, rowtab, rowtab_i, status);
 }
 
-inline dim3 row_grid(const Geometry& g, int bx) { return dim3((g.nx + bx - 1) / bx, g.ny, g.nz); }
 inline unsigned blocks_for(long long n, int b) { return (unsigned)((n + b - 1) / b); }
+inline unsigned node_grid(const Geometry& g, int b) { return blocks_for(g.N, b); }
+// node_at<true>: whole blocks to a row, and a grid within its limits
+inline bool rows_of_blocks(const Geometry& g, int b) {
+  return g.nx % b == 0 && g.ny <= 65535 && g.nz <= 65535;
+}
+inline dim3 row_grid(const Geometry& g, int b) { return dim3(g.nx / b, g.ny, g.nz); }
 
 }  // namespace
 
@@ -968,19 +960,19 @@ void launch_fused_step(const Geometry& g, const Rates& r, const T* fin, T* fout,
     if (fx) {
       if (!fcache || fnew.mode != FM_TABLE) fcache_mode = 0;
       if (g.channel)
-        k_fused<T, true, true><<<row_grid(g, B), B, 0, s>>>(g, rt, fin, fout, isnodes, fprev, fnew,
+        k_fused<T, true, true><<<node_grid(g, B), B, 0, s>>>(g, rt, fin, fout, isnodes, fprev, fnew,
                                                             fcache, fcache_mode);
       else
-        k_fused<T, false, true><<<row_grid(g, B), B, 0, s>>>(g, rt, fin, fout, isnodes, fprev, fnew,
+        k_fused<T, false, true><<<node_grid(g, B), B, 0, s>>>(g, rt, fin, fout, isnodes, fprev, fnew,
                                                              fcache, fcache_mode);
       count_launch();
       return;
     }
   }
   if (g.channel)
-    { k_fused<T, true><<<row_grid(g, B), B, 0, s>>>(g, rt, fin, fout, isnodes, fprev, fnew, nullptr, 0); count_launch(); }
+    { k_fused<T, true><<<node_grid(g, B), B, 0, s>>>(g, rt, fin, fout, isnodes, fprev, fnew, nullptr, 0); count_launch(); }
   else
-    { k_fused<T, false><<<row_grid(g, B), B, 0, s>>>(g, rt, fin, fout, isnodes, fprev, fnew, nullptr, 0); count_launch(); }
+    { k_fused<T, false><<<node_grid(g, B), B, 0, s>>>(g, rt, fin, fout, isnodes, fprev, fnew, nullptr, 0); count_launch(); }
 }
 
 void launch_fused_fixed(const Geometry& g, const Rates& r, bool int_core, const double* fin,
@@ -993,13 +985,17 @@ void launch_fused_fixed(const Geometry& g, const Rates& r, bool int_core, const 
   const long long* gi = reinterpret_cast<const long long*>(fin);
   long long* go = reinterpret_cast<long long*>(fout);
   long long* fci = reinterpret_cast<long long*>(fcache);
+  const bool ints = int_core && rt.int_ok, rows = ints && rows_of_blocks(g, B);
   auto launch = [&](auto kern) {
-    kern<<<row_grid(g, B), B, 0, s>>>(g, rt, gi, go, isnodes, fprev, fnew, fci, fcache_mode, st);
+    kern<<<rows ? row_grid(g, B) : dim3(node_grid(g, B)), B, 0, s>>>(g, rt, gi, go, isnodes, fprev,
+                                                                     fnew, fci, fcache_mode, st);
   };
-  if (int_core && rt.int_ok)
-    g.channel ? launch(k_fused_fixed<true, true>) : launch(k_fused_fixed<false, true>);
+  if (!ints)
+    g.channel ? launch(k_fused_fixed<true, false, false>) : launch(k_fused_fixed<false, false, false>);
+  else if (rows)
+    g.channel ? launch(k_fused_fixed<true, true, true>) : launch(k_fused_fixed<false, true, true>);
   else
-    g.channel ? launch(k_fused_fixed<true, false>) : launch(k_fused_fixed<false, false>);
+    g.channel ? launch(k_fused_fixed<true, true, false>) : launch(k_fused_fixed<false, true, false>);
   count_launch();
 }
 
@@ -1016,7 +1012,7 @@ template <typename T>
 void launch_macrovar(const Geometry& g, const T* f, const int32_t* isnodes,
                      const ForceView<T>& fv, const ParticleView& pv, T* rho, T* ux, T* uy,
                      T* uz, cudaStream_t s) {
-  { k_macrovar<T><<<row_grid(g, 128), 128, 0, s>>>(g, f, isnodes, fv, pv, rho, ux, uy, uz); count_launch(); }
+  { k_macrovar<T><<<node_grid(g, 128), 128, 0, s>>>(g, f, isnodes, fv, pv, rho, ux, uy, uz); count_launch(); }
 }
 
 template <typename T>
@@ -1026,12 +1022,12 @@ void launch_collision(const Geometry& g, const Rates& r, T* f, const int32_t* is
   const RatesT<double> rt = rates_t<double>(r);
   if constexpr (sizeof(T) == 8) {
     if (fx && rt.int_ok) {
-      k_collision<T, true><<<row_grid(g, 128), 128, 0, s>>>(g, r, rt, f, isnodes, fv, rho, ux, uy, uz);
+      k_collision<T, true><<<node_grid(g, 128), 128, 0, s>>>(g, r, rt, f, isnodes, fv, rho, ux, uy, uz);
       count_launch();
       return;
     }
   }
-  { k_collision<T><<<row_grid(g, 128), 128, 0, s>>>(g, r, rt, f, isnodes, fv, rho, ux, uy, uz); count_launch(); }
+  { k_collision<T><<<node_grid(g, 128), 128, 0, s>>>(g, r, rt, f, isnodes, fv, rho, ux, uy, uz); count_launch(); }
 }
 
 bool launch_relax(const Geometry& g, const Rates& r, const double* fin, double* fout,
@@ -1041,11 +1037,13 @@ bool launch_relax(const Geometry& g, const Rates& r, const double* fin, double* 
                   cudaStream_t s) {
   const RatesT<double> rt = rates_t<double>(r);
   if (!rt.int_ok) return false;
+  const bool rows = rows_of_blocks(g, 128);
   auto launch = [&](auto kern) {
-    kern<<<row_grid(g, 128), 128, 0, s>>>(g, r, rt, fin, fout, isnodes, fv, rho, ux, uy, uz, first,
-                                          before, change, eps);
+    kern<<<rows ? row_grid(g, 128) : dim3(node_grid(g, 128)), 128, 0, s>>>(
+        g, r, rt, fin, fout, isnodes, fv, rho, ux, uy, uz, first, before, change, eps);
   };
-  g.channel ? launch(k_relax<true>) : launch(k_relax<false>);
+  if (rows) g.channel ? launch(k_relax<true, true>) : launch(k_relax<false, true>);
+  else g.channel ? launch(k_relax<true, false>) : launch(k_relax<false, false>);
   count_launch();
   return true;
 }
@@ -1060,9 +1058,9 @@ void launch_rhoupdat_change(const Geometry& g, const double* f, double* rho,
 template <typename T>
 void launch_streaming(const Geometry& g, const T* fin, T* fout, cudaStream_t s) {
   if (g.channel)
-    { k_stream<T, true><<<row_grid(g, 128), 128, 0, s>>>(g, fin, fout); count_launch(); }
+    { k_stream<T, true><<<node_grid(g, 128), 128, 0, s>>>(g, fin, fout); count_launch(); }
   else
-    { k_stream<T, false><<<row_grid(g, 128), 128, 0, s>>>(g, fin, fout); count_launch(); }
+    { k_stream<T, false><<<node_grid(g, 128), 128, 0, s>>>(g, fin, fout); count_launch(); }
 }
 
 template <typename T>
@@ -1127,7 +1125,7 @@ void launch_convert_back(const T* in, double* out, long long n, cudaStream_t s) 
 template <typename T>
 void launch_force_field(const Geometry& g, const ForceView<T>& fv, double* fx, double* fy,
                         double* fz, cudaStream_t s) {
-  { k_force_field<T><<<row_grid(g, 128), 128, 0, s>>>(g, fv, fx, fy, fz); count_launch(); }
+  { k_force_field<T><<<node_grid(g, 128), 128, 0, s>>>(g, fv, fx, fy, fz); count_launch(); }
 }
 template <typename T>
 void launch_mass_momentum(const Geometry& g, const T* f, double* partial, int nblocks,
