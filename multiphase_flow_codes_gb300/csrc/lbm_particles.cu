@@ -100,9 +100,24 @@ __device__ Cands make_cands(double c, int n, double w, bool periodic) {
 }
 
 constexpr int MAXPLANES = 96;
-constexpr int MAXROWS = 640;   // processed rows per particle: (2 (rad + 2) + 1)^2
 constexpr int MAXC = 128;  // candidate positions per axis
-constexpr int MAXNEAR = 2048;  // fluid nodes within rad + 1.5 of one centre
+// Table sizes of the flag and link kernels: rows processed per particle,
+// (2 (rad + 2) + 1)^2, and fluid nodes within rad + 1.5 of its centre.  MANY:
+// spheres of up to kManyRad (225 rows; 637 nodes by volume) and more of them
+// than one wave of the large tables' blocks.  Their small tables let seven
+// blocks (flags; five, links) share an SM instead of four, and a flag thread
+// takes a row instead of a node, half the instructions but a longer chain
+// (256^3 FP32 with 1000 spheres: 0.612 -> 0.599 ms a step; with few spheres,
+// where the chain is what counts, 0.0853 -> 0.0866 at 32^3 with 5).
+constexpr double kManyRad = 5.0;
+constexpr int kManyBlocks = 4;  // resident per SM with the large tables
+bool many_spheres(const ParticleView& pv) {
+  return pv.rad <= kManyRad && pv.npart > kManyBlocks * sm_count();
+}
+template <bool MANY>
+constexpr int max_rows() { return MANY ? 256 : 640; }
+template <bool MANY>
+constexpr int max_near() { return MANY ? 768 : 2048; }
 
 // Sign decisions of the squared-distance tests of beads_links are taken in
 // FP32 when |value| exceeds this margin (the FP32 error is below 1e-4 for
@@ -383,7 +398,9 @@ __device__ __noinline__ bool inside_fp64(int i, int j, int k, double xc, double 
 // What beads_links' loop nest visits for one particle: candidate windows,
 // planes and rows with the image values in effect there, shared by the flag
 // and the link kernels.
+template <bool MANY, bool LINKS>
 struct LinkSetup {
+  static constexpr int MAXROWS = max_rows<MANY>();
   using Scan = cub::BlockScan<int, PB>;
   typename Scan::TempStorage scan_tmp;
   double par[5];  // radp2, rad2, x0, y0, z0
@@ -400,7 +417,7 @@ struct LinkSetup {
       float yyvf[3][MAXC];
       int plane_k[MAXPLANES];
     };
-    int16_t link_src[PB * 18];  // k_links: per link of the chunk, near node (local) << 5 | ipop
+    int16_t link_src[LINKS ? PB * 18 : 1];  // k_links: per link of the chunk, near node (local) << 5 | ipop
   };
   double xval[3][MAXC];
   float xofff[3][MAXC];  // (i - 1/2) - x centre per x candidate, FP64 then rounded
@@ -546,42 +563,71 @@ struct LinkSetup {
 
 // The solid nodes of one particle per block: all that the refill, and with it
 // the next stream + collide, needs of beads_links.  A thread takes node after
-// node of all rows.
+// node of all rows, or (MANY) a row: rows out of the sphere's reach end at
+// once, and a row's mask bits go out a word at a time.
+template <bool MANY>
 __device__ __forceinline__ void k_flags_body(int p, const Geometry& g, const ParticleView& pv, int32_t* isnodes,
                                               const LinkSlab& ls) {
-  __shared__ LinkSetup S;
+  __shared__ LinkSetup<MANY, false> S;
   if (p >= pv.npart) return;
   if (!S.fill(p, g, pv, ls)) return;
   const Cands& cx = S.cands[1];
-  const int tx = S.tx(), total = S.nrows * tx;
+  const int tx = S.tx();
   const float rad2f = S.parf[0], reachf = S.parf[1];
   const double rad2 = S.par[1];
   uint32_t* mask = const_cast<uint32_t*>(solid_mask(isnodes, g));
-  for (int t = threadIdx.x; t < total; t += PB) {
-    const int r = t / tx, ci = t - r * tx;
-    if (S.node_class(r, ci, rad2f, reachf, rad2) != 1) continue;
-    const int i = cx.at(ci), row = (S.row_k[r] - 1) * g.ny + (S.row_j[r] - 1);
-    atomicMax(&isnodes[(long long)row * g.nx + (i - 1)], p);
-    atomicOr(&mask[(size_t)row * g.sw + ((i - 1) >> 5)], 1u << ((i - 1) & 31));
+  if constexpr (MANY) {
+    for (int r = threadIdx.x; r < S.nrows; r += PB) {
+      const float yyf = S.row_yy[r], zzf = S.row_zz[r];
+      if (yyf * yyf + zzf * zzf - rad2f > kDecide) continue;
+      const int row = (S.row_k[r] - 1) * g.ny + (S.row_j[r] - 1);
+      int32_t* ids = isnodes + (long long)row * g.nx;
+      uint32_t* words = mask + (size_t)row * g.sw;
+      int ci = 0, word = 0;
+      uint32_t bits = 0;
+      for (int s = 0; s < cx.cnt; ++s)
+        for (int i = cx.lo[s] - 1; i < cx.hi[s] && ci < tx; ++i, ++ci) {
+          if (S.node_class(r, ci, rad2f, reachf, rad2) != 1) continue;
+          atomicMax(&ids[i], p);
+          if ((i >> 5) != word) {
+            if (bits) atomicOr(&words[word], bits);
+            word = i >> 5;
+            bits = 0;
+          }
+          bits |= 1u << (i & 31);
+        }
+      if (bits) atomicOr(&words[word], bits);
+    }
+  } else {
+    const int total = S.nrows * tx;
+    for (int t = threadIdx.x; t < total; t += PB) {
+      const int r = t / tx, ci = t - r * tx;
+      if (S.node_class(r, ci, rad2f, reachf, rad2) != 1) continue;
+      const int i = cx.at(ci), row = (S.row_k[r] - 1) * g.ny + (S.row_j[r] - 1);
+      atomicMax(&isnodes[(long long)row * g.nx + (i - 1)], p);
+      atomicOr(&mask[(size_t)row * g.sw + ((i - 1) >> 5)], 1u << ((i - 1) & 31));
+    }
   }
 }
-__global__ void __launch_bounds__(PB) k_flags(Geometry g, ParticleView pv, int32_t* isnodes, LinkSlab ls) {
-  k_flags_body(blockIdx.x, g, pv, isnodes, ls);
+template <bool MANY>
+__global__ void __launch_bounds__(PB, MANY ? 7 : 1) k_flags(Geometry g, ParticleView pv, int32_t* isnodes, LinkSlab ls) {
+  k_flags_body<MANY>(blockIdx.x, g, pv, isnodes, ls);
 }
 
 // The boundary links of one particle per block and what the bounce-back
 // needs of each: the next bounce-back is their first reader, so this runs
 // beside the refill and the next stream + collide.
-template <bool PREP>
+template <bool PREP, bool MANY>
 __device__ __forceinline__ void k_links_body(int p, const Geometry& g, const ParticleView& pv,
                                               const int32_t* __restrict__ isnodes, const LinkSlab& ls,
                                               DevStatus* st, int alpha_fp32) {
-  __shared__ LinkSetup S;
+  constexpr int MAXNEAR = max_near<MANY>();
+  __shared__ LinkSetup<MANY, true> S;
   __shared__ typename std::conditional<PREP, LeverTable<float>, int>::type levers;
   __shared__ int base;
   __shared__ int near_rc[MAXNEAR];  // fluid nodes within reach: row << 8 | candidate
   __shared__ int nnear;
-  using Scan = LinkSetup::Scan;
+  using Scan = typename LinkSetup<MANY, true>::Scan;
   if (p >= pv.npart) return;
   const int tid = threadIdx.x;
   if (tid == 0) { base = 0; nnear = 0; }
@@ -603,19 +649,23 @@ __device__ __forceinline__ void k_links_body(int p, const Geometry& g, const Par
   // per-row counts places each row's nodes.
   for (int r0 = 0; r0 < S.nrows; r0 += PB) {
     const int r = r0 + tid;
+    unsigned near[MAXC / 32];  // the row's nodes of class 2, a bit a candidate
     int cnt = 0;
-    if (r < S.nrows)
-      for (int ci = 0; ci < tx; ++ci) cnt += S.node_class(r, ci, rad2f, reachf, rad2) == 2;
+#pragma unroll
+    for (int h = 0; h < MAXC / 32; ++h) {
+      near[h] = 0;
+      if (r < S.nrows)
+        for (int ci = 32 * h; ci < min(tx, 32 * h + 32); ++ci)
+          near[h] |= (unsigned)(S.node_class(r, ci, rad2f, reachf, rad2) == 2) << (ci & 31);
+      cnt += __popc(near[h]);
+    }
     int pos, tot;
     Scan(S.scan_tmp).ExclusiveSum(cnt, pos, tot);
-    if (cnt) {
-      int w = nnear + pos;
-      for (int ci = 0; ci < tx; ++ci)
-        if (S.node_class(r, ci, rad2f, reachf, rad2) == 2) {
-          if (w < MAXNEAR) near_rc[w] = (r << 8) | ci;
-          ++w;
-        }
-    }
+    int w = nnear + pos;
+#pragma unroll
+    for (int h = 0; h < MAXC / 32; ++h)
+      for (unsigned m = near[h]; m; m &= m - 1, ++w)
+        if (w < MAXNEAR) near_rc[w] = (r << 8) | (32 * h + __ffs(m) - 1);
     __syncthreads();
     if (tid == 0) {
       if (nnear + tot > MAXNEAR) S.fixed_ok = 0;
@@ -784,14 +834,14 @@ __device__ __forceinline__ void k_links_body(int p, const Geometry& g, const Par
   if (tid == 0) {
     ls.count[p] = min(base, ls.cap);
     if (base > ls.cap) raise_error(st, LBM_ERR_CAPACITY, p);
-    if (S.nplanes >= MAXPLANES || S.nrows >= MAXROWS) raise_error(st, LBM_ERR_CAPACITY, p);
+    if (S.nplanes >= MAXPLANES || S.nrows >= max_rows<MANY>()) raise_error(st, LBM_ERR_CAPACITY, p);
     if (!S.fixed_ok) raise_error(st, LBM_ERR_STATE, p);
   }
 }
-template <bool PREP>
-__global__ void __launch_bounds__(PB) k_links(Geometry g, ParticleView pv, const int32_t* isnodes,
+template <bool PREP, bool MANY>
+__global__ void __launch_bounds__(PB, MANY ? 5 : 1) k_links(Geometry g, ParticleView pv, const int32_t* isnodes,
                                               LinkSlab ls, DevStatus* st, int alpha_fp32) {
-  k_links_body<PREP>(blockIdx.x, g, pv, isnodes, ls, st, alpha_fp32);
+  k_links_body<PREP, MANY>(blockIdx.x, g, pv, isnodes, ls, st, alpha_fp32);
 }
 
 // running sum: plain FP64, or FP32 with Kahan compensation (FP32 path)
@@ -1564,13 +1614,16 @@ int sm_count() {
 void launch_flags(const Geometry& g, const ParticleView& pv, int32_t* isnodes, LinkSlab ls,
                   cudaStream_t s) {
   if (pv.npart <= 0) return;
-  { k_flags<<<pv.npart, PB, 0, s>>>(g, pv, isnodes, ls); count_launch(); }
+  if (many_spheres(pv)) k_flags<true><<<pv.npart, PB, 0, s>>>(g, pv, isnodes, ls);
+  else k_flags<false><<<pv.npart, PB, 0, s>>>(g, pv, isnodes, ls);
+  count_launch();
 }
 void launch_link_lists(const Geometry& g, const ParticleView& pv, const int32_t* isnodes, LinkSlab ls,
                        DevStatus* st, int alpha_fp32, bool prep, cudaStream_t s) {
   if (pv.npart <= 0) return;
-  if (prep) k_links<true><<<pv.npart, PB, 0, s>>>(g, pv, isnodes, ls, st, alpha_fp32);
-  else k_links<false><<<pv.npart, PB, 0, s>>>(g, pv, isnodes, ls, st, alpha_fp32);
+  auto launch = [&](auto kern) { kern<<<pv.npart, PB, 0, s>>>(g, pv, isnodes, ls, st, alpha_fp32); };
+  if (prep) launch(k_links<true, false>);  // few spheres
+  else many_spheres(pv) ? launch(k_links<false, true>) : launch(k_links<false, false>);
   count_launch();
 }
 void launch_links(const Geometry& g, const ParticleView& pv, int32_t* isnodes, LinkSlab ls,
@@ -1717,12 +1770,12 @@ __global__ void k_reset_multi(const BoxParticles* boxes) {
 }
 __global__ void __launch_bounds__(PB) k_flags_multi(const BoxParticles* boxes) {
   BOX_OR_RETURN(B.pv.npart)
-  k_flags_body(blockIdx.x, B.g, B.pv, B.flags_next, B.ls);
+  k_flags_body<false>(blockIdx.x, B.g, B.pv, B.flags_next, B.ls);
 }
 template <bool PREP>
 __global__ void __launch_bounds__(PB) k_links_multi(const BoxParticles* boxes) {
   BOX_OR_RETURN(B.pv.npart)
-  k_links_body<PREP>(blockIdx.x, B.g, B.pv, B.flags_next, B.ls, B.st, 1);
+  k_links_body<PREP, false>(blockIdx.x, B.g, B.pv, B.flags_next, B.ls, B.st, 1);
 }
 __global__ void __launch_bounds__(PB) k_fill_detect_multi(const BoxParticles* boxes) {
   BOX_OR_RETURN(B.pv.npart)
