@@ -342,6 +342,19 @@ __host__ __device__ __forceinline__ double fx_to_k(long long v, int K) {
   memcpy(&d, &bits, 8);
   return a ? d : 0.0;
 }
+// fx_to_k with the device's own conversion (ties to even): one instruction of
+// the FP64 pipe and three others instead of ~20 integer ones, where that pipe
+// is idle (a pre-relaxation iteration at 128^3: 275 -> 233 us; with the
+// conversions to integers there too, 264).
+__host__ __device__ __forceinline__ double fx_to_cvt(long long v, int K) {
+#ifdef __CUDA_ARCH__
+  const double d = __ll2double_rn(v);
+  const int hi = __double2hiint(d);
+  return __hiloint2double(hi ? hi - (K << 20) : 0, __double2loint(d));
+#else
+  return fx_to_k(v, K);
+#endif
+}
 template <int K>
 __host__ __device__ __forceinline__ double fx_to(long long v) { return fx_to_k(v, K); }
 
@@ -826,9 +839,9 @@ __host__ __device__ __forceinline__ bool collide_fx_at(double (&f)[NPOP], bool s
                        split((long long)((unsigned long long)w[2] << j))};
   const long long rho_i = sum_rho ? o.rho : fx_from_k(rho, kFxIn + j);
   if (!fx_relax(o, rho_i, U, V, F, Fj, r, h, 0)) return false;
-  if (sum_rho) rho = fx_to_k(o.rho, kFxIn + j);
+  if (sum_rho) rho = fx_to_cvt(o.rho, kFxIn + j);
 #pragma unroll
-  for (int q = 0; q < NPOP; ++q) f[q] = fx_to_k(h[q], kFxOut + j);
+  for (int q = 0; q < NPOP; ++q) f[q] = fx_to_cvt(h[q], kFxOut + j);
   return true;
 }
 
