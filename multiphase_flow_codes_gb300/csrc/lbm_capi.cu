@@ -133,7 +133,8 @@ struct lbm_ctx {
   int npmax = 0, npart = 0;
   bool particles_on = false;
   double* pbuf = nullptr;  // 15 vectors of 3*npmax
-  double* part_host = nullptr;  // page-locked copy of pbuf for downloads
+  double* part_host = nullptr;  // page-locked copy of pbuf, from the second download on
+  bool part_downloaded = false;
   double *ypglb, *ypglbp, *wp, *wpp, *omgp, *omgpp, *dwdt, *domgdt, *forcep, *forcepp, *torqp,
       *torqpp, *thetap, *fHIp, *flubp;
   int* first_move = nullptr;
@@ -1847,12 +1848,13 @@ int lbm_download_particles(lbm_ctx* ctx, double* ypglb, double* wp, double* omgp
   double* outs[6] = {ypglb, wp, omgp, fHIp, flubp, torqp};
   double* srcs[6] = {ctx->ypglb, ctx->wp, ctx->omgp, ctx->fHIp, ctx->flubp, ctx->torqp};
   // All fifteen vectors lie in one buffer: one copy into page-locked memory
-  // (made on the first download) and the wanted ones from there, instead of a
-  // copy each into pageable arrays, which the driver stages and waits for
+  // (made on the second download: an allocation costs more than a download that
+  // stays the only one) and the wanted ones from there, instead of a copy each
+  // into pageable arrays, which the driver stages and waits for
   // (ten steps with a download each, FP32 32^3 with 5 spheres: 1.76 -> 1.23 ms;
   // FP64 64^3 with 16: 2.19 -> 1.69).
   const size_t v = 3 * (size_t)ctx->npmax;
-  if (!ctx->part_host &&
+  if (!ctx->part_host && ctx->part_downloaded &&
       cudaMallocHost((void**)&ctx->part_host, 15 * v * sizeof(double)) != cudaSuccess) {
     cudaGetLastError();
     ctx->part_host = nullptr;
@@ -1860,10 +1862,11 @@ int lbm_download_particles(lbm_ctx* ctx, double* ypglb, double* wp, double* omgp
   if (ctx->part_host)
     CK(cudaMemcpy2DAsync(ctx->part_host, v * sizeof(double), ctx->pbuf, v * sizeof(double), b, 15,
                          cudaMemcpyDeviceToHost, ctx->stream));
-  else  // no page-locked memory left
+  else
     for (int i = 0; i < 6; ++i)
       if (outs[i]) CK(cudaMemcpyAsync(outs[i], srcs[i], b, cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
+  ctx->part_downloaded = true;
   if (ctx->part_host)
     for (int i = 0; i < 6; ++i)
       if (outs[i]) std::memcpy(outs[i], ctx->part_host + (srcs[i] - ctx->pbuf), b);
