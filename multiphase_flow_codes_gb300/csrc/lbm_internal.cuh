@@ -387,6 +387,7 @@ constexpr int kPrepParticles = 304;  // two spheres an SM
 // launch_bounce_back's prep
 void launch_links(const Geometry& g, const ParticleView& pv, int32_t* isnodes,
                   LinkSlab ls, DevStatus* st, int alpha_fp32, bool prep, cudaStream_t s);
+void launch_clear_flags(const Geometry& g, int32_t* isnodes, int32_t* fill_count, cudaStream_t s);
 void launch_flags(const Geometry& g, const ParticleView& pv, int32_t* isnodes, LinkSlab ls,
                   cudaStream_t s);
 void launch_link_lists(const Geometry& g, const ParticleView& pv, const int32_t* isnodes, LinkSlab ls,
@@ -455,7 +456,7 @@ struct BoxParticles {
 // for nb boxes of the array, on s and aux; the caller waits for ev_links
 // before the next particle step
 void launch_particle_step_multi(const BoxParticles* boxes, int nb, int max_npart,
-                                long long max_reset, bool prep, cudaStream_t s, cudaStream_t aux,
+                                long long max_words, bool prep, cudaStream_t s, cudaStream_t aux,
                                 cudaEvent_t ev_fork, cudaEvent_t ev_join, cudaEvent_t ev_links);
 // FORCING of many boxes into table slot `slot`, keeping each box's state
 // before the update in `backup`
