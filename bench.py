@@ -478,8 +478,8 @@ def main():
         # from the ncu capture (FP64 only in the body-force series)
         fp64 = {"fp64_inst_per_node": figs[key].get("fp64_inst_per_node", 0.0),
                 "pipes_pct_of_peak": figs[key]["pipes"], "capture": figs[key].get("capture"),
-                "note": "integer collision core, FP64 body-force series: bound by the ALU pipe "
-                        "(fixed-point sums, 128-bit products, range tests), not by FP64 or HBM"}
+                "note": "integer collision core, FP64 body-force series: the heavy FMA pipe (32-bit "
+                        "products) and HBM close together; FP64 only in the force series"}
     elif dtype == "f64" and key in figs and figs[key].get("fp64_flop_per_node") and phases["stream_collide"][1]:
         sc_ms, sc_n = phases["stream_collide"]
         import ctypes as C
