@@ -463,9 +463,11 @@ __global__ void k_stream(Geometry g, const T* __restrict__ fin, T* __restrict__ 
 // the node's own scale (collide_fx_at), the literal FP64 form for the nodes it
 // declines.  The literal form's ~615 FP64 instructions a node took 1.75 ms at
 // 128^3, two thirds of a step of the subroutine loop there (150 spheres: 2.4
-// -> 0.69 ms a step with this and macrovar's integer sums).
+// -> 0.69 ms a step with this and macrovar's integer sums).  Five CTAs an SM
+// (96 registers, 156 bytes spilled) hide its loads best: that step without
+// spheres 427 us, four 447, six 432, three 468.
 template <typename T, bool FX = false>
-__global__ void __launch_bounds__(128, FX ? 4 : 1) k_collision(Geometry g, Rates r, RatesT<double> rt, T* __restrict__ f,
+__global__ void __launch_bounds__(128, FX ? 5 : 1) k_collision(Geometry g, Rates r, RatesT<double> rt, T* __restrict__ f,
                             const int32_t* __restrict__ isnodes, ForceView<T> fv,
                             const T* __restrict__ rho, const T* __restrict__ ux,
                             const T* __restrict__ uy, const T* __restrict__ uz) {
