@@ -948,6 +948,25 @@ __host__ __device__ __forceinline__ bool collide_fx_fixed_int(long long (&g)[NPO
   return true;
 }
 
+// A row of a force table (kRowCoef values, on a 16-byte boundary).  FP32: in
+// four 16-byte loads.  With the registers capped (k_fused) that leaves the
+// FP32 direct kernel with 9 loads a node for its two fields instead of 34
+// (box 250 x 251 x 249: 518 -> 467 us, 150 x 151 x 149: 148 -> 137; uncapped
+// it took 89 registers and 570 us).  In FP64 single loads are the faster
+// (256^3: 1.100 ms against 1.121).
+__device__ __forceinline__ void force_row(const float* __restrict__ p, float (&o)[kRowCoef]) {
+  const float4* v = reinterpret_cast<const float4*>(p);
+#pragma unroll
+  for (int i = 0; i < kRowCoef / 4; ++i) {
+    const float4 q = v[i];
+    o[4 * i] = q.x; o[4 * i + 1] = q.y; o[4 * i + 2] = q.z; o[4 * i + 3] = q.w;
+  }
+}
+__device__ __forceinline__ void force_row(const double* __restrict__ p, double (&o)[kRowCoef]) {
+#pragma unroll
+  for (int i = 0; i < kRowCoef - 1; ++i) o[i] = p[i];
+}
+
 // Body force of two fields (previous and current step) at one node, sharing
 // the per-x twiddles; see ForceView.
 template <typename T>
@@ -963,7 +982,8 @@ __device__ __forceinline__ void body_force2(const ForceView<T>& fa, const ForceV
   for (int w = 0; w < 2; ++w) {
     const ForceView<T>& v = *fv[w];
     if (v.mode == FM_TABLE) {
-      const T* k = v.rowtab + (long long)row * kRowCoef;
+      T k[kRowCoef];
+      force_row(v.rowtab + (long long)row * kRowCoef, k);
 #pragma unroll
       for (int c = 0; c < 3; ++c)
         out[w][c] = k[5 * c] + k[5 * c + 1] * c1 + k[5 * c + 2] * s1 + k[5 * c + 3] * c2 +

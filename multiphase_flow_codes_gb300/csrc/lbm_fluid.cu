@@ -215,7 +215,7 @@ __device__ __forceinline__ int wrapi(int i, int n) { return i < 0 ? i + n : (i >
 // step's field at every node (solid ones too: a node that becomes fluid
 // reads it next step).
 template <typename T, bool CHANNEL, bool FX = false>
-__global__ void __launch_bounds__(128, FX ? 4 : 1) k_fused(Geometry g, RatesT<T> r, const T* __restrict__ fin,
+__global__ void __launch_bounds__(128, FX ? 4 : (sizeof(T) == 4 ? 8 : 1)) k_fused(Geometry g, RatesT<T> r, const T* __restrict__ fin,
                                                T* __restrict__ fout,
                                                const int32_t* __restrict__ isnodes,
                                                ForceView<T> fprev, ForceView<T> fnew,
