@@ -869,7 +869,7 @@ uint64_t footprint(const lbm_config& c, int64_t* cap_out) {
   b += np * (uint64_t)cap * (4 + 8 + 8) + np * 4;
   if (es == 4) b += std::min<uint64_t>(np, kPrepParticles) * (uint64_t)cap * (3 + 6) * 4;
   b += np * (kSweepBytes + 3 * 4);                       // nearest-image sweeps
-  b += np * ((es == 8 ? 6ull * kBounceSplit * 8 : 0) + 4);  // bounce-back partial sums
+  if (es == 8) b += np * (6ull * kBounceSplit * 8 + 4);  // bounce-back partial sums
   if (np > 0) b += 2ull * std::max<uint64_t>(4096, 256 * np) * 4 + 4;  // refill list
   if (c.forcing == LBM_FORCING_STOCHASTIC) {
     b += 3ull * kRowCoef * c.ny * c.nz * es + 45ull * c.nz * 2 * 8;  // row tables, z table
@@ -1194,15 +1194,16 @@ int lbm_create(const lbm_config* cfg, lbm_ctx** out) {
     al((void**)&ctx->links.f9, (size_t)ctx->npmax * cap * sizeof(double));
     if (ctx->f32) {
       const size_t np = std::min(ctx->npmax, kPrepParticles);
-      al((void**)&ctx->links.gather, np * cap * 3 * sizeof(int32_t));
-      al((void**)&ctx->links.coef, np * cap * 6 * sizeof(float));
+      al((void**)&ctx->links.gather, np * cap * (3 * sizeof(int32_t) + 6 * sizeof(float)));
+      ctx->links.coef = reinterpret_cast<float*>(ctx->links.gather + np * cap * 3);
     }
     al((void**)&ctx->links.count, (size_t)ctx->npmax * sizeof(int32_t));
     al(&ctx->links.sweeps, (size_t)ctx->npmax * kSweepBytes);
     al((void**)&ctx->links.sweep_ok, (size_t)ctx->npmax * 3 * sizeof(int32_t));
-    if (!ctx->f32)
+    if (!ctx->f32) {
       al((void**)&ctx->links.bsum, (size_t)ctx->npmax * 6 * kBounceSplit * sizeof(double));
-    al((void**)&ctx->links.bdone, (size_t)ctx->npmax * sizeof(int32_t));
+      al((void**)&ctx->links.bdone, (size_t)ctx->npmax * sizeof(int32_t));
+    }
     ctx->fill.cap = std::max(4096, 256 * ctx->npmax);
     al((void**)&ctx->fill.node, (size_t)ctx->fill.cap * sizeof(int32_t));
     al((void**)&ctx->fill.part, (size_t)ctx->fill.cap * sizeof(int32_t));
@@ -1221,7 +1222,8 @@ int lbm_create(const lbm_config* cfg, lbm_ctx** out) {
     for (int i = 0; i < 15; ++i) *vecs[i] = b + i * v;
     cudaMemsetAsync(ctx->pbuf, 0, 15 * v * sizeof(double), ctx->stream);
     cudaMemsetAsync(ctx->links.count, 0, ctx->npmax * sizeof(int32_t), ctx->stream);
-    cudaMemsetAsync(ctx->links.bdone, 0, ctx->npmax * sizeof(int32_t), ctx->stream);
+    if (!ctx->f32)
+      cudaMemsetAsync(ctx->links.bdone, 0, ctx->npmax * sizeof(int32_t), ctx->stream);
     cudaMemsetAsync(ctx->first_move, 0, sizeof(int), ctx->stream);
   }
   cudaMemsetAsync(ctx->f[0], 0, 19 * N * ctx->esz, ctx->stream);
@@ -1334,7 +1336,7 @@ int lbm_destroy(lbm_ctx* ctx) {
                   ctx->rowtab[2], ctx->pbuf, ctx->first_move, ctx->links.code,
                   ctx->links.alpha, ctx->links.f9, ctx->links.count, ctx->links.sweeps,
                   ctx->links.sweep_ok, ctx->links.bsum, ctx->links.bdone,
-                  ctx->links.gather, ctx->links.coef, ctx->fill.node,
+                  ctx->links.gather, ctx->fill.node,
                   ctx->fill.part, ctx->fill.count, ctx->fcache, ctx->xtw_i,
                   ctx->rowtab_i[0], ctx->rowtab_i[1], ctx->rowtab_i[2]};
   for (void* p : ptrs)
