@@ -810,12 +810,18 @@ __host__ __device__ __forceinline__ bool fx_core_int(const long long (&g)[NPOP],
 // collision_MRT of FP64 populations with the density and velocity given (its
 // own subroutine takes them from macrovar's arrays), in the integer core at a
 // scale of the node's own: 2^j finer than fx_core_int's, with the largest j
-// for which populations, velocity, density and force stay in its ranges, so
-// that 54 bits and more below the node's largest population are kept (FP64
-// has 53 below each).  sum_rho: the density is the populations' sum (rho is
-// set to it).  False, with f as it was, when a value is not finite or too
-// large, or the node is so quiet that j would pass 40 (its populations below
-// 2^-44): the caller then takes the FP64 form.
+// for which populations, velocity, density and force stay in its ranges.
+// sum_rho: the density is the populations' sum (rho is set to it).  False,
+// with f as it was, when a value is not finite or too large, when the node is
+// so quiet that j would pass 40 (its populations below 2^-44), or when
+// velocity, density or force would lower j by more than kFxYield below the
+// populations' own scale, each step of which costs them a bit: the caller then
+// takes the FP64 form.  An equilibrium's velocity lowers j by one at most; a
+// force does from a hundredth of the velocity on (a flow started from rest by
+// its body force).  Error against 128-bit floating point, relative to the
+// node's largest population, rms / max: j lowered by 0 or 1 1.4e-16 / 3.3e-16
+// (FP64 form 2.0e-16 / 5.6e-16), by 2 2.6e-16 / 5.0e-16, by 4 9e-16 / 2.6e-15.
+constexpr int kFxYield = 1;
 __host__ __device__ __forceinline__ bool collide_fx_at(double (&f)[NPOP], bool sum_rho, double& rho,
                                                        double ux, double uy, double uz, double fx,
                                                        double fy, double fz,
@@ -828,24 +834,22 @@ __host__ __device__ __forceinline__ bool collide_fx_at(double (&f)[NPOP], bool s
   const int eF = most(fx_exponent(fx), most(fx_exponent(fy), fx_exponent(fz)));
   // |f| < 2^(-4 - j), |u| < 2^(-2 - j), |F| < 2^(-9 - j), |rho| < 2^(-1 - j)
   // as fixed point: 2^54, 2^62, 2^61, 2^57
-  int j = 1018 - ef;
-  j = -most(-j, most(eu - 1020, eF - 1013));
+  const int jf = 1018 - ef;
+  int j = -most(-jf, most(eu - 1020, eF - 1013));
   if (!sum_rho) j = -most(-j, fx_exponent(rho) - 1021);
-  if (j < 0 || j > 40) return false;
+  if (j < 0 || j > 40 || jf - j > kFxYield) return false;
   long long g[NPOP], h[NPOP];
 #pragma unroll
   for (int q = 0; q < NPOP; ++q) g[q] = fx_from_k(f[q], kFxIn + j);
   FxSums o;
   fx_sums(g, o);
   const long long u[3] = {fx_from_k(ux, kFxUU + j), fx_from_k(uy, kFxUU + j), fx_from_k(uz, kFxUU + j)};
-  const long long w[3] = {fx_from_k(fx, kFxF), fx_from_k(fy, kFxF), fx_from_k(fz, kFxF)};
+  const long long w[3] = {fx_from_k(fx, kFxF + j), fx_from_k(fy, kFxF + j), fx_from_k(fz, kFxF + j)};
   const long long half = (1LL << j) >> 1;
   const Split U[3] = {split(u[0]), split(u[1]), split(u[2])};
   const Split V[3] = {split((u[0] + half) >> j), split((u[1] + half) >> j), split((u[2] + half) >> j)};
-  const Split F[3] = {split(w[0]), split(w[1]), split(w[2])};
-  const Split Fj[3] = {split((long long)((unsigned long long)w[0] << j)),
-                       split((long long)((unsigned long long)w[1] << j)),
-                       split((long long)((unsigned long long)w[2] << j))};
+  const Split Fj[3] = {split(w[0]), split(w[1]), split(w[2])};
+  const Split F[3] = {split((w[0] + half) >> j), split((w[1] + half) >> j), split((w[2] + half) >> j)};
   const long long rho_i = sum_rho ? o.rho : fx_from_k(rho, kFxIn + j);
   if (!fx_relax(o, rho_i, U, V, F, Fj, r, h, 0)) return false;
   if (sum_rho) rho = fx_to_cvt(o.rho, kFxIn + j);
