@@ -55,23 +55,26 @@ constexpr int kFxUU = 64;                   // velocities and u_a u_b inside fx_
 // finer for the two that the inverse transform multiplies by up to 30 and 12.
 __host__ __device__ constexpr int kFxM(int k) { return k == 1 ? 63 : (k == 2 ? 62 : kFxOut); }
 // The integer core sums the products of a moment at the scale
-// 2^-(kFxM(k) + kFxS(k)) and rounds the sum once, by a shift of kFxS(k).  64
-// takes the high word as it is; the moments whose factor on the populations
-// is larger than 2^-4 (|A_k| <= c_k: 1/12 for 8, 1/4 for 10..12, 1/8 for
-// 13..15) need a smaller one so that the factor fits 63 bits.
-__host__ __device__ constexpr int kFxS(int k) {
-  return k == 8 || k >= 13 ? 63 : (k >= 10 ? 62 : 64);
+// 2^-(kFxM(k) + 64) and rounds the sum once, to its high word.  The factor on the
+// populations must fit 63 bits (|A_k| <= c_k: 1/12 for 8, 1/4 for 10..12, 1/8 for
+// 13..15): these moments' sums, which are small ones, are raised by kFxUp(k)
+// bits instead, exactly.  (With a smaller shift of the sum in its place the
+// products of the low words, which dot_shift leaves out, count for half a unit
+// and more: error of the stress moments 0.61 -> 0.69 units of 2^-58 at rates
+// near 2, and adding them takes 2.5 % of a step.)
+__host__ __device__ constexpr int kFxUp(int k) {
+  return k == 8 || k >= 13 ? 1 : (k >= 10 ? 2 : 0);
 }
 // scale of factor i of RatesT::Ch: that of its moment's sum over that of the
 // value it multiplies
 __host__ __device__ constexpr int kFxSc(int i) {
-  if (i <= 15) return kFxM(i) + kFxS(i) - kFxIn;              // A_k ev_k
-  if (i <= 18) return kFxM(i - 15) + kFxS(i - 15) - kFxIn;    // B1r, B2r, 1/19 times rho
+  if (i <= 15) return kFxM(i) + 64 - kFxIn - kFxUp(i);     // A_k ev_k
+  if (i <= 18) return kFxM(i - 15) + 64 - kFxIn;           // B1r, B2r, 1/19 times rho
   // velocity terms at 2^-kFxUU (even), force terms at 2^-kFxF (odd); the
   // momentum's last two at the scales of moment 3
   const int n = i - 19, sv = (n & 1) ? kFxF : kFxUU;
   const int k = n < 2 ? 1 : n < 4 ? 2 : n < 6 ? 3 : n < 14 ? 6 + (n - 6) / 2 : n < 16 ? 10 : 3;
-  return kFxM(k) + kFxS(k) - sv;
+  return kFxM(k) + 64 - sv;
 }
 
 // c as (integer m, shift sh) with c = m * 2^-sh exactly and |m| in
@@ -700,41 +703,38 @@ __host__ __device__ __forceinline__ bool fx_relax(const FxSums& o, long long rho
   auto N = [&](int k) { return C(19 + k); };
   I M[16];
   // a moment of the populations, a velocity term and a force term
-  auto moment = [&](auto S, int k, I ev, Split v, int nv, Split w, int nw) {
-    const Split x[3] = {split(ev), v, w}, y[3] = {C(k), N(nv), N(nw)};
-    return dot_shift<decltype(S)::value, 3>(x, y);
+  auto moment = [&](int k, Split v, int nv, Split w, int nw) {
+    const Split x[3] = {split(o.ev[k] * (1 << kFxUp(k))), v, w}, y[3] = {C(k), N(nv), N(nw)};
+    return dot_shift<64, 3>(x, y);
   };
   // moments 1 and 2 also hold a density term
   auto moment_rho = [&](int k, I ev, Split v, int nv, Split w, int nw) {
     const Split x[4] = {split(ev), rhos, v, w}, y[4] = {C(k), C(15 + k), N(nv), N(nw)};
-    return dot_shift<kFxS(1), 4>(x, y);
+    return dot_shift<64, 4>(x, y);
   };
-  auto alone = [&](int k, I ev) {
-    const Split x[1] = {split(ev)}, y[1] = {C(k)};
-    return dot_shift<kFxS(13), 1>(x, y);
+  auto alone = [&](int k) {
+    const Split x[1] = {split(o.ev[k] * (1 << kFxUp(k)))}, y[1] = {C(k)};
+    return dot_shift<64, 1>(x, y);
   };
   auto momentum = [&](int a) {
     const Split x[2] = {U[a], Fj[a]}, y[2] = {N(16), N(17)};
     return dot_shift<64, 2>(x, y);
   };
-  const std::integral_constant<int, kFxS(3)> s64{};
-  const std::integral_constant<int, kFxS(8)> s8{};
-  const std::integral_constant<int, kFxS(10)> s10{};
   M[1] = moment_rho(1, o.ev[1], t1, 0, G3, 1);
   M[2] = moment_rho(2, o.ev[2], t1, 2, G3, 3);
-  M[3] = moment(s64, 3, o.ev[3], U[0], 4, Fj[0], 5);
-  M[4] = moment(s64, 4, o.ev[4], U[1], 4, Fj[1], 5);
-  M[5] = moment(s64, 5, o.ev[5], U[2], 4, Fj[2], 5);
-  M[6] = moment(s64, 6, o.ev[6], eq6, 6, e6, 7);
-  M[7] = moment(s64, 7, o.ev[7], eq6, 8, e6, 9);
-  M[8] = moment(s8, 8, o.ev[8], eq8, 10, e8, 11);
-  M[9] = moment(s64, 9, o.ev[9], eq8, 12, e8, 13);
-  M[10] = moment(s10, 10, o.ev[10], qxy, 14, m10, 15);
-  M[11] = moment(s10, 11, o.ev[11], qyz, 14, m11, 15);
-  M[12] = moment(s10, 12, o.ev[12], qxz, 14, m12, 15);
-  M[13] = alone(13, o.ev[13]);
-  M[14] = alone(14, o.ev[14]);
-  M[15] = alone(15, o.ev[15]);
+  M[3] = moment(3, U[0], 4, Fj[0], 5);
+  M[4] = moment(4, U[1], 4, Fj[1], 5);
+  M[5] = moment(5, U[2], 4, Fj[2], 5);
+  M[6] = moment(6, eq6, 6, e6, 7);
+  M[7] = moment(7, eq6, 8, e6, 9);
+  M[8] = moment(8, eq8, 10, e8, 11);
+  M[9] = moment(9, eq8, 12, e8, 13);
+  M[10] = moment(10, qxy, 14, m10, 15);
+  M[11] = moment(11, qyz, 14, m11, 15);
+  M[12] = moment(12, qxz, 14, m12, 15);
+  M[13] = alone(13);
+  M[14] = alone(14);
+  M[15] = alone(15);
   const Split xr[1] = {rhos}, yr[1] = {C(18)};
   const I tl1 = dot_shift<64, 1>(xr, yr);
   const I tl6 = momentum(0), tl8 = momentum(1), tl10 = momentum(2);

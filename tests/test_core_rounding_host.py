@@ -45,6 +45,16 @@ def test_mean_error_is_the_last_roundings(rows):
             assert abs(mean) <= 1 / 16 + 0.003, (mrt, visc, mean)
 
 
+def test_stress_error_is_the_populations_roundings(rows):
+    """The stress c_x c_y f sums four populations' roundings to the storage, 0.577
+    units, and its moment's own at 1/8 unit, entering fourfold: a rounding and
+    three products without their low words, 0.32 units rms, 0.16; 0.6 in all."""
+    for mrt, visc, int_ok, states, declined, mean, rms, xy in step_rows(rows):
+        if int_ok:
+            # (rms of 20000 states: to 0.5 %)
+            assert xy <= 0.62, (mrt, visc, xy)
+
+
 def test_no_mass_at_a_nodes_own_scale(rows):
     """Populations are rounded to the node's scale and its results to FP64, ties
     to even: no mean error beyond five standard errors of 20000 states whose
