@@ -41,7 +41,8 @@ struct RatesT {
   // all-integer core (fx_core_int), each at the scale 2^kFxSc[i] as
   // Ch * 2^32 + Cl with a signed low word (|Cl| <= 2^31): [0..18] as Li,
   // [19..36] B1t H1 B2t H2 B3 H3 B6 H6 B7 H7 B8 H8 B9 H9 B10 H10 0.1 0.05.
-  // int_ok: every factor fits its scale (any rates in (0, 2) do)
+  // int_ok: every factor fits its scale (rates that are 2^-31 or more from the
+  // ends of (0, 2) do: viscosities from 2e-11 on)
   int Ch[37], Cl[37];
   bool int_ok;
 };
@@ -120,7 +121,7 @@ RatesT<T> rates_t(const Rates& r) {
                    : i == 16 ? -11.0 * Bk(1) : i == 17 ? r.omegepsl * Bk(2)
                    : i == 18 ? 1.0 / 19.0 : nf[i - 19];
     const double v = std::ldexp(c, kFxSc(i));
-    const bool fits = std::fabs(v) < 9.2e18;  // below 2^63 - 2^31
+    const bool fits = std::fabs(v) < 0x1p63 - 0x1p31;  // Ch in 32 bits
     o.int_ok = o.int_ok && fits;
     const long long m = fits ? (long long)std::llround(v) : 0;
     o.Cl[i] = (int)(unsigned)(unsigned long long)m;
@@ -615,9 +616,10 @@ __host__ __device__ __forceinline__ long long dot_shift(const Split (&a)[n], con
 // each moment is one sum of products of such values and fixed-point factors
 // (RatesT::Ch), rounded once to 2^-kFxOut.  Ranges, so that nothing
 // overflows: |u| < 2^-2 and |F| < 2^-9 (a node beyond them is declined, as
-// is one whose moments leave their ranges).  With |g| < 2^55 the largest sum
-// of middle terms is M1's: below 8.6e18 (the linear program over all inputs
-// with |u_a| < 2^-2, and low words of 2^31) against 2^63 = 9.2e18.
+// is one whose moments leave their ranges).  With |g| < 2^55, low words of 2^31
+// and any rates in (0, 2) the largest sum of middle terms is M1's: below 9.1e18
+// (ev_1 and rho together 197 2^55: 3.55e18, rho's low word 2.7e18 at a rate of
+// 2, t1 1.8e18, G3 0.9e18, ev_1's low word 0.1e18) against 2^63 = 9.22e18.
 //
 // bias is added to every output (through tl1, which each of them holds once):
 // the caller's rounding constant costs one add instead of nineteen.

@@ -55,6 +55,17 @@ def test_stress_error_is_the_populations_roundings(rows):
             assert xy <= 0.62, (mrt, visc, xy)
 
 
+def test_rates_near_two_keep_the_integer_core(rows):
+    """Every rate set down to viscosities of 1e-8 (rates within 1e-7 of 2) has
+    factors that fit their scales, and near-equilibrium nodes are taken with the
+    error of the core: a rounding to the storage, 0.29 units, and the moments'
+    roundings at 1/8 unit, less than 0.3 in all."""
+    for mrt, visc, int_ok, states, declined, mean, rms, xy in step_rows(rows):
+        assert int_ok == 1, (mrt, visc)
+        assert declined == 0, (mrt, visc)
+        assert rms <= (0.29 ** 2 + 0.3 ** 2) ** 0.5, (mrt, visc, rms)
+
+
 def test_no_mass_at_a_nodes_own_scale(rows):
     """Populations are rounded to the node's scale and its results to FP64, ties
     to even: no mean error beyond five standard errors of 20000 states whose
