@@ -310,7 +310,8 @@ enum {
  * STAGED in FP32, else DIRECT. */
 int lbm_set_variant(lbm_ctx* ctx, int variant, int stages, int groups, int ctas_per_sm);
 int lbm_get_variant(lbm_ctx* ctx, int* variant, int* stages, int* groups, int* ctas_per_sm);
-/* Arithmetic of the collision in the fused stream + collide kernels.
+/* Arithmetic of the collision in the fused stream + collide kernels, and of
+ * collision_MRT, macrovar and the pre-relaxation (below).
  * LBM_SUMS_FLOAT: every operation in the populations' precision.
  * LBM_SUMS_FIXED (FP64 contexts): the sums with small integer coefficients
  * of the forward and inverse moment transforms are computed exactly in
@@ -328,8 +329,17 @@ int lbm_get_variant(lbm_ctx* ctx, int* variant, int* stages, int* groups, int* c
  * that stays in range (|u| < 1/4, |F| < 2^-9; others take the FP64 path);
  * the body-force series is evaluated in FP64 beside it and rounded once to
  * its fixed point.
- * FP32 contexts accept LBM_SUMS_FLOAT only.  The unfused per-subroutine
- * entries always use LBM_SUMS_FLOAT.  No counterpart in the reference. */
+ * The per-subroutine entries and the unfused step keep FP64 populations of
+ * any magnitude.  With LBM_SUMS_INTEGER lbm_collision_mrt and lbm_prerelax
+ * take the integer collision at a scale of each node's own (2^j finer, its
+ * largest population at the top of the range); a node whose velocity, density
+ * or force would lower that scale by more than a bit, whose populations are
+ * all below 2^-44 or beyond 1/16, or that is not finite takes the FP64 form.
+ * With the other two they collide in FP64.  lbm_macrovar sums density and
+ * momentum exactly in integers at such a scale, except with LBM_SUMS_FLOAT,
+ * which keeps every operation FP64.  The integer forms' errors are no larger
+ * than the FP64 forms'.
+ * FP32 contexts accept LBM_SUMS_FLOAT only.  No counterpart in the reference. */
 enum { LBM_SUMS_FLOAT = 0, LBM_SUMS_FIXED = 1, LBM_SUMS_INTEGER = 2 };
 int lbm_set_sums(lbm_ctx* ctx, int mode);
 int lbm_get_sums(lbm_ctx* ctx, int* mode);

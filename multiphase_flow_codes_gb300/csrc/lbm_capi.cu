@@ -433,7 +433,7 @@ template <typename T>
 void materialize_macro_t(lbm_ctx* c) {
   launch_macrovar<T>(c->g, fbuf<T>(c, c->cur), c->flags[c->fcur], fview<T>(c, c->fmacro),
                      pview(c), mbuf<T>(c, 0), mbuf<T>(c, 1), mbuf<T>(c, 2), mbuf<T>(c, 3),
-                     c->stream);
+                     c->sums != LBM_SUMS_FLOAT, c->stream);
 }
 void materialize_macro(lbm_ctx* c) {
   if (!c->macro_pending) return;
@@ -830,7 +830,7 @@ void unfused_step_t(lbm_ctx* c) {
   do_forcing(c);
   launch_collision<T>(c->g, c->r, fbuf<T>(c, c->cur), c->flags[c->fcur], fview<T>(c, c->latest),
                       mbuf<T>(c, 0), mbuf<T>(c, 1), mbuf<T>(c, 2), mbuf<T>(c, 3),
-                      c->sums != LBM_SUMS_FLOAT, c->stream);
+                      c->sums == LBM_SUMS_INTEGER, c->stream);
   if (c->particles_on) {
     join_links(c);
     launch_bounce_back<T>(c->g, pview(c), fbuf<T>(c, c->cur), 0, c->flags[c->fcur], c->links,
@@ -1971,7 +1971,7 @@ int lbm_collision_mrt(lbm_ctx* ctx) {
     launch_collision<double>(ctx->g, ctx->r, fbuf<double>(ctx, ctx->cur), ctx->flags[ctx->fcur],
                              fview<double>(ctx, ctx->latest), mbuf<double>(ctx, 0),
                              mbuf<double>(ctx, 1), mbuf<double>(ctx, 2), mbuf<double>(ctx, 3),
-                             ctx->sums != LBM_SUMS_FLOAT, ctx->stream);
+                             ctx->sums == LBM_SUMS_INTEGER, ctx->stream);
   ctx->macro_derived = false;
   CK(cudaGetLastError());
   return LBM_OK;
@@ -2141,7 +2141,7 @@ int lbm_prerelax(lbm_ctx* ctx, double eps, int max_iter, int* iters, double* err
   if (ctx->in_batch) return fail(ctx, LBM_ERR_STATE, "a batched context steps only through its batch");
   materialize_macro(ctx);
   // (max_iter + 2 must not overflow; such a count takes the loop below)
-  if (!ctx->f32 && ctx->sums != LBM_SUMS_FLOAT && max_iter < (1 << 30)) {
+  if (!ctx->f32 && ctx->sums == LBM_SUMS_INTEGER && max_iter < (1 << 30)) {
     const int rc = prerelax_passes(ctx, eps, max_iter, iters, err);
     if (rc <= 0) return rc;
   }

@@ -581,8 +581,9 @@ __global__ void __launch_bounds__(128, 4) k_relax(Geometry g, Rates r, RatesT<do
 }
 
 // macrovar, B/collision.f90:232-332 (solid branch with nearest image; the
-// channel has no x image, C/collision.f90:294-295)
-template <typename T>
+// channel has no x image, C/collision.f90:294-295).  FX (FP64): exact integer
+// sums (fx_moments)
+template <typename T, bool FX = false>
 __global__ void k_macrovar(Geometry g, const T* __restrict__ f,
                            const int32_t* __restrict__ isnodes, ForceView<T> fv,
                            ParticleView pv, T* __restrict__ rho, T* __restrict__ ux,
@@ -595,7 +596,7 @@ __global__ void k_macrovar(Geometry g, const T* __restrict__ f,
   for (int q = 0; q < NPOP; ++q) fl[q] = f[q * N + n];
   T rho9, ux9, uy9, uz9, fx, fy, fz;
   bool done = false;
-  if constexpr (sizeof(T) == 8) done = fx_moments(fl, rho9, ux9, uy9, uz9);
+  if constexpr (FX) done = fx_moments(fl, rho9, ux9, uy9, uz9);
   if (!done) moments(fl, rho9, ux9, uy9, uz9);
   body_force(fv, g, x, y, z, fx, fy, fz);
   T u1 = ux9 + fx * T(0.5), u2 = uy9 + fy * T(0.5), u3 = uz9 + fz * T(0.5), rr = rho9;
@@ -1013,8 +1014,13 @@ void launch_pop_format(double* f, long long n, bool to_fixed, DevStatus* st, cud
 template <typename T>
 void launch_macrovar(const Geometry& g, const T* f, const int32_t* isnodes,
                      const ForceView<T>& fv, const ParticleView& pv, T* rho, T* ux, T* uy,
-                     T* uz, cudaStream_t s) {
-  { k_macrovar<T><<<node_grid(g, 128), 128, 0, s>>>(g, f, isnodes, fv, pv, rho, ux, uy, uz); count_launch(); }
+                     T* uz, bool fx, cudaStream_t s) {
+  auto launch = [&](auto kern) {
+    kern<<<node_grid(g, 128), 128, 0, s>>>(g, f, isnodes, fv, pv, rho, ux, uy, uz);
+  };
+  if constexpr (sizeof(T) == 8) fx ? launch(k_macrovar<T, true>) : launch(k_macrovar<T>);
+  else launch(k_macrovar<T>);
+  count_launch();
 }
 
 template <typename T>
@@ -1178,7 +1184,7 @@ void launch_forcing_tables(const Geometry& g, const ForcingDev* st, const T* ytw
                                      const ForceView<T>&, bool, T*, int, cudaStream_t);     \
   template void launch_macrovar<T>(const Geometry&, const T*, const int32_t*,               \
                                    const ForceView<T>&, const ParticleView&, T*, T*, T*, T*, \
-                                   cudaStream_t);                                           \
+                                   bool, cudaStream_t);                                     \
   template void launch_collision<T>(const Geometry&, const Rates&, T*, const int32_t*,      \
                                     const ForceView<T>&, const T*, const T*, const T*,      \
                                     const T*, bool, cudaStream_t);                          \

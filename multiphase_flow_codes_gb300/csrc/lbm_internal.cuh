@@ -241,10 +241,12 @@ void launch_fused_batch(bool channel, const BatchBox* boxes, const BatchTask* ta
                         const BatchPhase& ph, const Rates& r, const StagedPlan& p, DevStatus* st,
                         cudaStream_t s);
 
+// fx (FP64): sums (macrovar) or the whole collision in integer arithmetic, for
+// the nodes that it can take
 template <typename T>
 void launch_macrovar(const Geometry& g, const T* f, const int32_t* isnodes,
                      const ForceView<T>& fv, const ParticleView& pv, T* rho, T* ux,
-                     T* uy, T* uz, cudaStream_t s);
+                     T* uy, T* uz, bool fx, cudaStream_t s);
 template <typename T>
 void launch_collision(const Geometry& g, const Rates& r, T* f, const int32_t* isnodes,
                       const ForceView<T>& fv, const T* rho, const T* ux, const T* uy,
