@@ -73,6 +73,7 @@ struct lbm_ctx {
   cudaEvent_t ev_links = nullptr;
   bool links_pending = false;
   bool links_prep = false;  // the link lists hold the bounce-back's gathers too
+  bool links_moved = false;  // spheres moved since the lists were built (beads_move by itself)
   bool aux_pending = false;
   bool store_pending = false;  // the bounce-back stores run on aux until ev_store
   bool prefetched = false;
@@ -545,7 +546,16 @@ void join_links(lbm_ctx* c) {
 bool want_prep(const lbm_ctx* c) { return c->f32 && c->npart <= kPrepParticles; }
 void links_now(lbm_ctx* c, int32_t* flags) {
   c->links_prep = want_prep(c);
+  c->links_moved = false;
   launch_links(c->g, pview(c), flags, c->links, c->status, c->f32 ? 1 : 0, c->links_prep, c->stream);
+}
+
+// Spheres moved without new link lists: the lists still say which links there
+// are, but the lever arms formed with them are those of the old centres, and
+// the next bounce-back forms its own.
+void spheres_moved(lbm_ctx* c) {
+  c->links_prep = false;
+  c->links_moved = true;
 }
 
 // The part of the particle step that reads no post-collision populations:
@@ -601,6 +611,7 @@ void particle_phase(lbm_ctx* c, T* f_plain) {
   cudaEventRecord(c->ev_aux_fork, c->stream);
   cudaStreamWaitEvent(c->aux, c->ev_aux_fork, 0);
   c->links_prep = want_prep(c);
+  c->links_moved = false;
   launch_link_lists(c->g, pview(c), c->flags[nf], c->links, c->status, c->f32 ? 1 : 0, c->links_prep,
                     c->aux);
   cudaEventRecord(c->ev_links, c->aux);
@@ -780,6 +791,7 @@ void graph_step_t(lbm_ctx* c) {
     g_launches.fetch_add(g.kernels);
     for (int s = 0; s < 3; ++s) c->slot_version[s] += g.slot_writes[s];
     set_step_state(c, g.after);
+    c->links_moved = false;
     c->fcache_version = c->fcache_slot >= 0 ? c->slot_version[c->fcache_slot] : 0;
     c->macro_pending = true;
     c->macro_derived = true;
@@ -2020,6 +2032,7 @@ int lbm_beads_move(lbm_ctx* ctx) {
   if (!ctx) return LBM_ERR_ARG;
   if (!ctx->particles_on) return LBM_OK;
   launch_move(ctx->g, ctx->npart, ctx->pp, mstate(ctx), ctx->stream);
+  spheres_moved(ctx);
   CK(cudaGetLastError());
   return LBM_OK;
 }
@@ -2028,6 +2041,7 @@ int lbm_beads_redistribute(lbm_ctx* ctx) {
   if (!ctx) return LBM_ERR_ARG;
   if (!ctx->particles_on) return LBM_OK;
   launch_redistribute(ctx->g, ctx->npart, ctx->pp, mstate(ctx), ctx->status, ctx->stream);
+  spheres_moved(ctx);
   CK(cudaGetLastError());
   return check_status(ctx);
 }
@@ -2537,6 +2551,7 @@ std::string batch_step_eager(lbm_batch* b) {
     c->macro_pending = true;
     c->macro_derived = true;
     c->links_prep = b->prep;
+    c->links_moved = false;
   }
   return "";
 }
@@ -2571,10 +2586,15 @@ int lbm_batch_create(lbm_ctx** ctxs, int n, lbm_batch** out) {
     c->in_batch = true;
     c->fcache_slot = -1;
   }
-  // few spheres in all: lists with the gathers, also those built before
+  // few spheres in all: lists with the gathers, also those built before (of
+  // spheres that have not moved since)
   long long spheres = 0;
-  for (lbm_ctx* c : b->ctx) spheres += c->particles_on ? c->npart : 0;
-  b->prep = spheres > 0 && spheres <= kPrepParticles;
+  bool moved = false;
+  for (lbm_ctx* c : b->ctx) {
+    spheres += c->particles_on ? c->npart : 0;
+    moved = moved || (c->particles_on && c->links_moved);
+  }
+  b->prep = spheres > 0 && spheres <= kPrepParticles && !moved;
   for (lbm_ctx* c : b->ctx)
     if (b->prep && c->particles_on && !c->links_prep) {
       launch_link_lists(c->g, pview(c), c->flags[c->fcur], c->links, c->status, 1, true, c->stream);
