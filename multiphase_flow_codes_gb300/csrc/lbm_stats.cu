@@ -819,7 +819,7 @@ int fluid_rms_stats(const Geometry& g, const int32_t* isnodes, const T* ux, cons
         cudaStreamSynchronize(s) != cudaSuccess)
       return LBM_ERR_CUDA;
     for (int k = 0; k < 3; ++k) {
-      om[k] = 0.0;
+      om[k] = std::isnan(h[k]) ? h[k] : 0.0;  // (a field that is not finite has no mean)
       orr[k] = sqrt(h[k] / ((double)N * (double)N));  // N^2 < 2^53: exact
     }
   } else {
