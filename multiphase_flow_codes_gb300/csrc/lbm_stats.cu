@@ -585,16 +585,18 @@ static void fold(SpectrumWork* w, long long n, int K, double* out, cudaStream_t 
 }
 
 // the forward transforms of three fields.  FP64 fields on 16-byte boundaries
-// (an even N) are read where they lie, others through a copy.
+// are read where they lie, others through a copy.  The transforms take no field
+// off such a boundary, which the second of three fields of an odd N is: such
+// boxes have no spectrum.
 template <typename T>
 static int forward(SpectrumWork* w, const T* const (&u)[3], long long N, long long nc, cudaStream_t s) {
+  if (N % 2) return LBM_ERR_CUDA;
   cufftSetStream(w->fwd, s);
   for (int a = 0; a < 3; ++a) {
     double* in = w->real + a * N;
     if (sizeof(T) == 8 && reinterpret_cast<uintptr_t>(u[a]) % 16 == 0) {
       in = reinterpret_cast<double*>(const_cast<T*>(u[a]));  // D2Z keeps its input
     } else {
-      if (N % 2) in = w->real;  // one after the other, on a boundary
       k_to_double<T><<<blocks(N, 256), 256, 0, s>>>(u[a], in, N);
       count_launch();
     }
