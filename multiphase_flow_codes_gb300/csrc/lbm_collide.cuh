@@ -894,7 +894,7 @@ __host__ __device__ __forceinline__ bool collide_fx_at(double (&f)[NPOP], bool s
 // of the node's own (the largest population at 2^58, so nothing below 2^-58 of
 // it is lost), rounded once: 4 conversions back instead of the ~40 FP64 adds
 // that bound macrovar on this GPU's FP64 pipe.  False for values that are not
-// finite or all below 2^-900.
+// finite, large enough for a sum beyond FP64's range, or all below 2^-900.
 __host__ __device__ __forceinline__ bool fx_moments(const double (&f)[NPOP], double& rho, double& jx,
                                                     double& jy, double& jz) {
   int ef = 0;
@@ -903,7 +903,7 @@ __host__ __device__ __forceinline__ bool fx_moments(const double (&f)[NPOP], dou
     const int e = fx_exponent(f[q]);
     ef = ef > e ? ef : e;
   }
-  if (ef >= 2047 || ef < 123) return false;
+  if (ef >= 2047 - 5 || ef < 123) return false;  // (19 of them: 2^5 times the largest)
   const int K = 1022 + 58 - ef;
   long long g[NPOP];
 #pragma unroll
