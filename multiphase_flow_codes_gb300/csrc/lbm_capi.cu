@@ -22,6 +22,8 @@ using namespace lbm;
 namespace {
 
 std::atomic<long long> g_launches{0};
+// those of this thread, which a captured graph's kernels are counted by
+thread_local long long t_launches = 0;
 
 constexpr int kStagingDoubles = 1 << 25;  // 256 MB chunk for host transfers
 
@@ -158,7 +160,10 @@ struct lbm_ctx {
 };
 
 namespace lbm {
-void count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
+void count_launch() {
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  ++t_launches;
+}
 }
 
 namespace {
@@ -802,7 +807,7 @@ void graph_step_t(lbm_ctx* c) {
   const unsigned long long fv = c->fcache_version;
   unsigned long long versions[3];
   std::memcpy(versions, c->slot_version, sizeof versions);
-  const int64_t l0 = g_launches.load();
+  const long long l0 = t_launches;
   if (cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeRelaxed) == cudaSuccess) {
     fused_step_t<T>(c);
     join_links(c);
@@ -814,7 +819,7 @@ void graph_step_t(lbm_ctx* c) {
     ok = ok && cudaGraphInstantiate(&g.exec, gr, 0) == cudaSuccess;
     if (gr) cudaGraphDestroy(gr);
     if (ok) {
-      g.kernels = g_launches.load() - l0;
+      g.kernels = t_launches - l0;
       g.after = step_state(c);
       for (int s = 0; s < 3; ++s) g.slot_writes[s] = (int)(c->slot_version[s] - versions[s]);
       if (cudaGraphLaunch(g.exec, c->stream) == cudaSuccess) {
@@ -826,6 +831,7 @@ void graph_step_t(lbm_ctx* c) {
   }
   // no graph: nothing has run, so the step is made as it stands
   cudaGetLastError();
+  g_launches.fetch_sub(t_launches - l0);
   c->graphs_off = true;
   set_step_state(c, before);
   c->fcache_version = fv;
@@ -2762,7 +2768,7 @@ int lbm_batch_step(lbm_batch* b, int nsteps, int use_graph) {
           cudaGraphExecDestroy(b->graph);
           b->graph = nullptr;
         }
-        const int64_t l0 = g_launches.load();
+        const long long l0 = t_launches;
         BK(cudaStreamBeginCapture(b->main, cudaStreamCaptureModeRelaxed));
         std::string err;
         for (int k = 0; k < kBatchCycle && err.empty(); ++k) err = batch_step_eager(b);
@@ -2779,7 +2785,7 @@ int lbm_batch_step(lbm_batch* b, int nsteps, int use_graph) {
         cudaError_t e = cudaGraphInstantiate(&b->graph, gr, 0);
         cudaGraphDestroy(gr);
         BK(e);
-        b->graph_kernels = g_launches.load() - l0;
+        b->graph_kernels = t_launches - l0;
         for (int i = 0; i < kKey; ++i) b->graph_key[i] = key[i];
         // capturing advanced the host state by one cycle; the replay below
         // performs that cycle on the device
