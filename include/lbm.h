@@ -473,6 +473,11 @@ int lbm_profile(lbm_ctx* ctx, int enable);
 int lbm_profile_read(lbm_ctx* ctx, int phase, double* ms_total, int64_t* count);
 /* number of kernels this library has launched in this process */
 int64_t lbm_kernel_launches(void);
+/* number of lbm_step's steps that ran as a captured graph so far: single steps
+ * that find their stream idle, in boxes with spheres and up to 2^21 nodes,
+ * after some hundreds of fused steps.  They leave the same bits as directly
+ * launched ones. */
+int lbm_replayed_steps(const lbm_ctx* ctx, int64_t* steps);
 /* Measured FMA throughput (TFLOP/s, an FMA counted as 2 flops) of the
  * current device in FP64 (precision = LBM_PREC_F64) or FP32: the compute
  * roofline of the fused kernel.  No counterpart in the reference. */

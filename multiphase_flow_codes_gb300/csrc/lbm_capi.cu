@@ -84,7 +84,7 @@ struct lbm_ctx {
   // captured steps (graph_step) and the fused steps made so far
   std::vector<StepGraph> graphs;
   bool graphs_off = false;
-  int64_t fused_steps = 0;
+  int64_t fused_steps = 0, replayed_steps = 0;
   ForcingDev* d_forcing_backup = nullptr;
   bool status_pending = false;
   std::string err;
@@ -795,6 +795,7 @@ void graph_step_t(lbm_ctx* c) {
     if (cudaGraphLaunch(g.exec, c->stream) != cudaSuccess) break;
     g_launches.fetch_add(g.kernels);
     for (int s = 0; s < 3; ++s) c->slot_version[s] += g.slot_writes[s];
+    ++c->replayed_steps;
     set_step_state(c, g.after);
     c->links_moved = false;
     c->fcache_version = c->fcache_slot >= 0 ? c->slot_version[c->fcache_slot] : 0;
@@ -823,6 +824,7 @@ void graph_step_t(lbm_ctx* c) {
       g.after = step_state(c);
       for (int s = 0; s < 3; ++s) g.slot_writes[s] = (int)(c->slot_version[s] - versions[s]);
       if (cudaGraphLaunch(g.exec, c->stream) == cudaSuccess) {
+        ++c->replayed_steps;
         c->graphs.push_back(g);
         return;
       }
@@ -2376,6 +2378,12 @@ int lbm_profile_read(lbm_ctx* ctx, int phase, double* ms_total, int64_t* count) 
 }
 
 int64_t lbm_kernel_launches(void) { return g_launches.load(); }
+
+int lbm_replayed_steps(const lbm_ctx* ctx, int64_t* steps) {
+  if (!ctx || !steps) return LBM_ERR_ARG;
+  *steps = ctx->replayed_steps;
+  return LBM_OK;
+}
 
 int lbm_mass_momentum(lbm_ctx* ctx, double out[4]) {
   if (!ctx || !out) return LBM_ERR_ARG;

@@ -110,6 +110,12 @@ class LBMBox:
             out[name] = (ms.value, int(n.value))
         return out
 
+    def replayed_steps(self) -> int:
+        """Steps of step(1) so far that ran as a captured graph."""
+        n = C.c_int64(0)
+        self._ck(self._L.lbm_replayed_steps(self._h, C.byref(n)), "replayed_steps")
+        return n.value
+
     @staticmethod
     def kernel_launches() -> int:
         return int(capi.lib().lbm_kernel_launches())
