@@ -455,14 +455,18 @@ int lbm_server_destroy(lbm_server* server);
  * sum c f. */
 int lbm_mass_momentum(lbm_ctx* ctx, double out[4]);
 
-/* Device time per phase of the time step, from CUDA events recorded on the
- * context's stream around each phase.  enable = 1 clears the totals and
- * starts recording, 0 stops.  Phases (LBM_PHASE_*): */
+/* Device time per phase of the time step, from CUDA events recorded around
+ * each phase on the stream that runs it.  FORCING and, in a fused step, the
+ * link lists run beside other phases (so the phases can add up to more than
+ * the step), as do the clearing of the flags, beads_lubforce, the overlap check
+ * and the bounce-back's stores, which no phase times.  enable = 1 clears the
+ * totals and starts recording, 0 stops.  Phases (LBM_PHASE_*): */
 enum {
   LBM_PHASE_STREAM_COLLIDE = 0, /* fused stream + MRT collide (or the unfused kernels) */
-  LBM_PHASE_BOUNCE = 1,         /* beads_collision: bounce-back + stores              */
-  LBM_PHASE_PARTICLES = 2,      /* beads_lubforce, beads_move, beads_redistribute     */
-  LBM_PHASE_LINKS = 3,          /* beads_links (flag reset + link build)              */
+  LBM_PHASE_BOUNCE = 1,         /* beads_collision: bounce-back                       */
+  LBM_PHASE_PARTICLES = 2,      /* beads_move, beads_redistribute's wrap, image sweeps */
+  LBM_PHASE_LINKS = 3,          /* beads_links: an interval for the solid flags and one
+                                   for the link lists                                 */
   LBM_PHASE_FILLING = 4,        /* beads_filling                                      */
   LBM_PHASE_FORCING = 5,        /* FORCING (state update + force tables)              */
   LBM_NPHASES = 6

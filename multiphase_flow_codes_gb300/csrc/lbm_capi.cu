@@ -618,8 +618,14 @@ void particle_phase(lbm_ctx* c, T* f_plain) {
   cudaStreamWaitEvent(c->aux, c->ev_aux_fork, 0);
   c->links_prep = want_prep(c);
   c->links_moved = false;
+  size_t l0 = 0, l1 = 0;
+  if (c->prof_on) cudaEventRecord(next_event(c, &l0), c->aux);
   launch_link_lists(c->g, pview(c), c->flags[nf], c->links, c->status, c->f32 ? 1 : 0, c->links_prep,
                     c->aux);
+  if (c->prof_on) {
+    cudaEventRecord(next_event(c, &l1), c->aux);
+    c->intervals.push_back({LBM_PHASE_LINKS, l0, l1});
+  }
   cudaEventRecord(c->ev_links, c->aux);
   c->links_pending = true;
   prof_end(c, LBM_PHASE_LINKS);
