@@ -2379,6 +2379,7 @@ int lbm_profile(lbm_ctx* ctx, int enable) {
 int lbm_profile_read(lbm_ctx* ctx, int phase, double* ms_total, int64_t* count) {
   if (!ctx || phase < 0 || phase >= LBM_NPHASES) return LBM_ERR_ARG;
   CK(cudaStreamSynchronize(ctx->stream));
+  CK(cudaStreamSynchronize(ctx->side));  // the next step's FORCING
   double tot = 0.0;
   int64_t n = 0;
   for (const auto& iv : ctx->intervals) {

@@ -25,3 +25,14 @@ def test_intervals_of_a_step(require_gpu, prec):
     box.profile(False)
     box.step(3)
     assert box.profile_read()["links"][1] == 2 * steps
+
+
+def test_read_while_the_next_forcing_runs(require_gpu):
+    """Without spheres a small step ends before the next step's FORCING, which is
+    timed on its own stream."""
+    box = make_box(16, 0, 3.0, 61)
+    box.profile(True)
+    for k in range(200):
+        box.step(1)
+        # (the first FORCING runs in the step itself and is not timed)
+        assert box.profile_read()["forcing"][1] >= k
