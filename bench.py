@@ -430,7 +430,7 @@ def main():
         cfg_desc["collision_sums"] = {
             "fixed": "integer-coefficient moment sums exact in 64-bit fixed point, products FP64",
             "integer": "moment sums exact in 64-bit fixed point, velocity and force products as "
-                       "exact 128-bit integer products; body-force series in FP64, rounded once to "
+                       "integer products in 32-bit halves; body-force series in FP64, rounded once to "
                        "fixed point",
             "float": "all FP64"}[args.sums]
 

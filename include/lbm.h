@@ -201,8 +201,9 @@ int lbm_rhoupdat(lbm_ctx* ctx);           /* collision.f90:213 rhoupdat       */
  * 71-95): repeat collision_MRT, streaming, rhoupdat with the velocity held
  * fixed until max|rho - rho_previous| <= eps or the iteration counter passes
  * max_iter (the reference: rhoepsl = 1e-5, 15000).  iters: the counter at
- * exit (the reference's printed istep); err: the last max difference.  One
- * 8-byte read-back per iteration. */
+ * exit (the reference's printed istep); err: the last max difference.  With
+ * LBM_SUMS_INTEGER one kernel an iteration, and the differences are read back
+ * sixteen at a time; otherwise three, and one read-back per iteration. */
 int lbm_prerelax(lbm_ctx* ctx, double eps, int max_iter, int* iters, double* err);
 
 /* The whole time step of main.f90:172-188, `nsteps` times, fused into a
@@ -323,9 +324,10 @@ int lbm_get_variant(lbm_ctx* ctx, int* variant, int* stages, int* groups, int* c
  * about 1/32 of its 32-bit integer rate, and these sums are most of the FP64
  * kernel's instructions.
  * LBM_SUMS_INTEGER (FP64 contexts, their default): LBM_SUMS_FIXED with the
- * velocity and force terms as exact 128-bit integer products of fixed-point
- * values too (products rounded once to 2^-64 or 2^-70, each term of a moment
- * once to 2^-61), so the collision issues no FP64 instruction on a node
+ * velocity and force terms as integer products of fixed-point values too
+ * (products rounded once to 2^-64 or 2^-70; each moment one sum of products
+ * by signed 32-bit halves, without those of the low words, rounded once to
+ * 2^-61 or finer), so the collision issues no FP64 instruction on a node
  * that stays in range (|u| < 1/4, |F| < 2^-9; others take the FP64 path);
  * the body-force series is evaluated in FP64 beside it and rounded once to
  * its fixed point.

@@ -742,11 +742,14 @@ void fused_step_t(lbm_ctx* c) {
 // little) and replays it: the same calls, with both side streams joined at the
 // end.  Ten steps with a download each, FP32 32^3 with 5 spheres 1.23 -> 1.03
 // ms, FP64 64^3 with 16 1.69 -> 1.60; FP32 128^3 with 150 0.203 -> 0.177 ms a
-// step.  Only for a single step that finds the stream idle, and up to
-// kGraphNodes (FP64 128^3 0.294 -> 0.272 ms): where steps are queued ahead of
-// the device, direct launches leave the host out of the way and keep the side
-// streams' overlap with the next step, which the joins end (64^3 with 16:
-// 0.095 ms a step against 0.105; 128^3 FP32 with 150: 0.150 against 0.161).
+// step (FP64 0.294 -> 0.272).  Only for a single step that finds the stream
+// idle: where steps are queued ahead of the device, direct launches leave the
+// host out of the way and keep the side streams' overlap with the next step,
+// which the joins end (64^3 with 16: 0.095 ms a step against 0.105; 128^3 FP32
+// with 150: 0.150 against 0.161).  kGraphNodes is the size that the replays are
+// tested up to and not where their gain ends (direct against replayed, step and
+// wait: 160^3 with 300 FP32 0.262 and 0.240 ms, FP64 0.439 and 0.424; 256^3 with
+// 1000 0.627 and 0.608, 1.385 and 1.359).
 constexpr long long kGraphNodes = 1LL << 21;
 
 StepState step_state(const lbm_ctx* c) {

@@ -381,8 +381,9 @@ __host__ __device__ __forceinline__ double fx_to_k(long long v, int K) {
 }
 // fx_to_k with the device's own conversion (ties to even): one instruction of
 // the FP64 pipe and three others instead of ~20 integer ones, where that pipe
-// is idle (a pre-relaxation iteration at 128^3: 275 -> 233 us; with the
-// conversions to integers there too, 264).
+// is idle (a pre-relaxation iteration at 128^3 303 -> 249 us, an unfused step
+// 488 -> 458; with the conversions to integers there too, 264 against 233 when
+// it came).
 __host__ __device__ __forceinline__ double fx_to_cvt(long long v, int K) {
 #ifdef __CUDA_ARCH__
   const double d = __ll2double_rn(v);
@@ -609,20 +610,6 @@ __host__ __device__ __forceinline__ long long dot_shift(const Split (&a)[n], con
 #endif
 }
 
-// fx_core with the velocity and force terms as integer products too, so the
-// collision issues no FP64 instruction: the velocity u (scale 2^-kFxIn, then
-// 2^-kFxUU) and this step's body force F (2^-kFxF) enter as integers; the
-// products u_a u_b are rounded once to 2^-kFxUU and F_a u_b to 2^-kFxF, and
-// each moment is one sum of products of such values and fixed-point factors
-// (RatesT::Ch), rounded once to 2^-kFxOut.  Ranges, so that nothing
-// overflows: |u| < 2^-2 and |F| < 2^-9 (a node beyond them is declined, as
-// is one whose moments leave their ranges).  With |g| < 2^55, low words of 2^31
-// and any rates in (0, 2) the largest sum of middle terms is M1's: below 9.1e18
-// (ev_1 and rho together 197 2^55: 3.55e18, rho's low word 2.7e18 at a rate of
-// 2, t1 1.8e18, G3 0.9e18, ev_1's low word 0.1e18) against 2^63 = 9.22e18.
-//
-// bias is added to every output (through tl1, which each of them holds once):
-// the caller's rounding constant costs one add instead of nineteen.
 // The integer sums of the forward transform (collision.f90:101-118): density,
 // momentum and the moments ev_1..ev_15 of the populations g.
 struct FxSums { long long rho, jx, jy, jz, ev[16]; };
@@ -809,6 +796,20 @@ __host__ __device__ __forceinline__ bool fx_relax(const FxSums& o, long long rho
   return true;
 }
 
+// fx_core with the velocity and force terms as integer products too, so the
+// collision issues no FP64 instruction: the velocity u (scale 2^-kFxIn, then
+// 2^-kFxUU) and this step's body force F (2^-kFxF) enter as integers; the
+// products u_a u_b are rounded once to 2^-kFxUU and F_a u_b to 2^-kFxF, and
+// each moment is one sum of products of such values and fixed-point factors
+// (RatesT::Ch), rounded once to 2^-kFxOut.  Ranges, so that nothing
+// overflows: |u| < 2^-2 and |F| < 2^-9 (a node beyond them is declined, as
+// is one whose moments leave their ranges).  With |g| < 2^55, low words of 2^31
+// and any rates in (0, 2) the largest sum of middle terms is M1's: below 9.1e18
+// (ev_1 and rho together 197 2^55: 3.55e18, rho's low word 2.7e18 at a rate of
+// 2, t1 1.8e18, G3 0.9e18, ev_1's low word 0.1e18) against 2^63 = 9.22e18.
+//
+// bias is added to every output (through tl1, which each of them holds once):
+// the caller's rounding constant costs one add instead of nineteen.
 __host__ __device__ __forceinline__ bool fx_core_int(const long long (&g)[NPOP], long long fpx,
                                                      long long fpy, long long fpz, long long Fx,
                                                      long long Fy, long long Fz,

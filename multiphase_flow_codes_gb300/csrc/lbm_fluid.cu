@@ -350,8 +350,8 @@ __device__ __forceinline__ void body_force_fxd(const ForceView<double>& fv, cons
 // cache (fcache_mode as in k_fused) holds them as 64-bit integers at 2^-kFxF.
 // Five CTAs of 128 threads per SM (96 registers): the integer core is now
 // short enough that loads and stores bound it, and more warps hide them
-// (256^3 with 1000 spheres: 1.01 ms, 5.0 TB/s of populations; four CTAs at
-// 128 registers 1.11 ms, three 1.24 ms, six 1.02 ms; before, with 128-bit
+// (256^3 with 1000 spheres: 1.05 ms, 4.9 TB/s of populations; four CTAs at
+// 128 registers 1.12 ms, three 1.25 ms, six 1.06 ms; before, with 128-bit
 // products, 1.54 ms at four).
 template <bool CHANNEL, bool INTCORE, bool ROWS>
 __global__ void __launch_bounds__(128, 5) k_fused_fixed(Geometry g, RatesT<double> r,
@@ -463,9 +463,9 @@ __global__ void k_stream(Geometry g, const T* __restrict__ fin, T* __restrict__ 
 // the node's own scale (collide_fx_at), the literal FP64 form for the nodes it
 // declines.  The literal form's ~615 FP64 instructions a node took 1.75 ms at
 // 128^3, two thirds of a step of the subroutine loop there (150 spheres: 2.4
-// -> 0.69 ms a step with this and macrovar's integer sums).  Five CTAs an SM
-// (96 registers, 156 bytes spilled) hide its loads best: that step without
-// spheres 427 us, four 447, six 432, three 468.
+// -> 0.71 ms a step with this and macrovar's integer sums).  Five CTAs an SM
+// (96 registers, 260 bytes spilled) hide its loads best: that step without
+// spheres 458 us, four 474, six 480, three 504.
 template <typename T, bool FX = false>
 __global__ void __launch_bounds__(128, FX ? 5 : 1) k_collision(Geometry g, Rates r, RatesT<double> rt, T* __restrict__ f,
                             const int32_t* __restrict__ isnodes, ForceView<T> fv,
@@ -501,7 +501,8 @@ __global__ void __launch_bounds__(128, FX ? 5 : 1) k_collision(Geometry g, Rates
 // populations as they stand with the largest density change of the iteration
 // that made them, then the next iteration's collision_MRT (velocity held) and
 // streaming into the other buffer: 2 x 19 + 5 values a node instead of the
-// 2 x 42 + 20 of three kernels (128^3: 1.96 -> 0.27 ms).
+// 2 x 42 + 20 of three kernels (128^3: 1.96 -> 0.249 ms; three CTAs an SM 0.253,
+// five 0.291).
 // first: the collision uses the stored density (no iteration made these
 // populations).  before: the change the previous pass found; when it is within
 // eps or not finite the loop has ended, and this pass does nothing.
