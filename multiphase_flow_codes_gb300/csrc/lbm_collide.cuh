@@ -43,13 +43,16 @@ struct RatesT {
   // [19..36] B1t H1 B2t H2 B3 H3 B6 H6 B7 H7 B8 H8 B9 H9 B10 H10 0.1 0.05.
   // int_ok: every factor fits its scale (rates that are 2^-31 or more from the
   // ends of (0, 2) do: viscosities from 2e-11 on)
-  int Ch[37], Cl[37];
+  // Wh, Wl: the force terms' factors (H1, H2, .., H10, 0.05) again, for forces at
+  // 2^-kFxWide
+  int Ch[37], Cl[37], Wh[9], Wl[9];
   bool int_ok;
 };
 
 constexpr int kFxIn = 58, kFxInMax = -3;    // inputs, forward transform
 constexpr int kFxOut = 61, kFxOutMax = -5;  // scaled moments, inverse transform
 constexpr int kFxF = 70;                    // body forces: |F| < 2^-7 at 2^-70
+constexpr int kFxWide = 64;                 // body forces of collide_fx_at, times 2^j
 constexpr int kFxUU = 64;                   // velocities and u_a u_b inside fx_core_int
 
 // Scale 2^-kFxM(k) of the scaled moment k in the integer core: kFxOut, but
@@ -68,12 +71,12 @@ __host__ __device__ constexpr int kFxUp(int k) {
 }
 // scale of factor i of RatesT::Ch: that of its moment's sum over that of the
 // value it multiplies
-__host__ __device__ constexpr int kFxSc(int i) {
+__host__ __device__ constexpr int kFxSc(int i, int force = kFxF) {
   if (i <= 15) return kFxM(i) + 64 - kFxIn - kFxUp(i);     // A_k ev_k
   if (i <= 18) return kFxM(i - 15) + 64 - kFxIn;           // B1r, B2r, 1/19 times rho
-  // velocity terms at 2^-kFxUU (even), force terms at 2^-kFxF (odd); the
+  // velocity terms at 2^-kFxUU (even), force terms at 2^-force (odd); the
   // momentum's last two at the scales of moment 3
-  const int n = i - 19, sv = (n & 1) ? kFxF : kFxUU;
+  const int n = i - 19, sv = (n & 1) ? force : kFxUU;
   const int k = n < 2 ? 1 : n < 4 ? 2 : n < 6 ? 3 : n < 14 ? 6 + (n - 6) / 2 : n < 16 ? 10 : 3;
   return kFxM(k) + 64 - sv;
 }
@@ -120,12 +123,17 @@ RatesT<T> rates_t(const Rates& r) {
     const double c = i < 16 ? ck[i] * (1.0 - sk[i])
                    : i == 16 ? -11.0 * Bk(1) : i == 17 ? r.omegepsl * Bk(2)
                    : i == 18 ? 1.0 / 19.0 : nf[i - 19];
-    const double v = std::ldexp(c, kFxSc(i));
-    const bool fits = std::fabs(v) < 0x1p63 - 0x1p31;  // Ch in 32 bits
-    o.int_ok = o.int_ok && fits;
-    const long long m = fits ? (long long)std::llround(v) : 0;
-    o.Cl[i] = (int)(unsigned)(unsigned long long)m;
-    o.Ch[i] = (int)((m - o.Cl[i]) >> 32);
+    auto factor = [&](int sc, int& hi, int& lo) {
+      const double v = std::ldexp(c, sc);
+      const bool fits = std::fabs(v) < 0x1p63 - 0x1p31;  // hi in 32 bits
+      o.int_ok = o.int_ok && fits;
+      const long long m = fits ? (long long)std::llround(v) : 0;
+      lo = (int)(unsigned)(unsigned long long)m;
+      hi = (int)((m - lo) >> 32);
+    };
+    factor(kFxSc(i), o.Ch[i], o.Cl[i]);
+    const int n = i - 19;
+    if (n >= 0 && (n & 1)) factor(kFxSc(i, kFxWide), o.Wh[n / 2], o.Wl[n / 2]);
   }
   return o;
 }
@@ -659,10 +667,11 @@ __host__ __device__ __forceinline__ void fx_sums(const long long (&g)[NPOP], FxS
 
 // Relaxation and inverse transform on the sums of one node.  Everything is
 // at the scales of fx_core_int times 2^j: rho (2^-(kFxIn + j)), the velocity U
-// (2^-(kFxUU + j)) and the force Fj (2^-(kFxF + j)); V and F are the velocity
-// and the force at 2^-kFxUU and 2^-kFxF (U and Fj themselves for j = 0), so
-// that the products u_a u_b and F_a u_b are at 2^j times their scales too.
-// False when a moment leaves its range.
+// (2^-(kFxUU + j)) and the force Fj (2^-(kFxF + j), WIDE: 2^-(kFxWide + j)); V and
+// F are the velocity and the force without the 2^j (U and Fj themselves for
+// j = 0), so that the products u_a u_b and F_a u_b are at 2^j times their scales
+// too.  False when a moment leaves its range.
+template <bool WIDE>
 __host__ __device__ __forceinline__ bool fx_relax(const FxSums& o, long long rho, const Split (&U)[3],
                                                   const Split (&V)[3], const Split (&F)[3],
                                                   const Split (&Fj)[3], const RatesT<double>& r,
@@ -689,7 +698,9 @@ __host__ __device__ __forceinline__ bool fx_relax(const FxSums& o, long long rho
   const Split m12 = split(mul2(F[0], U[2], F[2], U[0]));
   const Split rhos = split(rho);
   auto C = [&](int i) { return Split{r.Ch[i], r.Cl[i]}; };
-  auto N = [&](int k) { return C(19 + k); };
+  auto N = [&](int k) {
+    return WIDE && (k & 1) ? Split{r.Wh[k / 2], r.Wl[k / 2]} : C(19 + k);
+  };
   I M[16];
   // a moment of the populations, a velocity term and a force term
   auto moment = [&](int k, Split v, int nv, Split w, int nw) {
@@ -837,7 +848,7 @@ __host__ __device__ __forceinline__ bool fx_core_int(const long long (&g)[NPOP],
   constexpr int su = kFxUU - kFxIn;
   const Split U[3] = {split(ux << su), split(uy << su), split(uz << su)};
   const Split F[3] = {split(Fx), split(Fy), split(Fz)};
-  return fx_relax(o, o.rho, U, U, F, F, r, h, bias);
+  return fx_relax<false>(o, o.rho, U, U, F, F, r, h, bias);
 }
 
 // collision_MRT of FP64 populations with the density and velocity given (its
@@ -849,10 +860,12 @@ __host__ __device__ __forceinline__ bool fx_core_int(const long long (&g)[NPOP],
 // so quiet that j would pass 40 (its populations below 2^-44), or when
 // velocity, density or force would lower j by more than kFxYield below the
 // populations' own scale, each step of which costs them a bit: the caller then
-// takes the FP64 form.  An equilibrium's velocity lowers j by one at most; a
-// force does from a hundredth of the velocity on (a flow started from rest by
-// its body force).  Error against 128-bit floating point, relative to the
-// node's largest population, rms / max: j lowered by 0 or 1 1.4e-16 / 3.3e-16
+// takes the FP64 form.  An equilibrium's velocity lowers j by one at most, a
+// force from twice the largest population on (its scale is kFxWide and not
+// kFxF: at that one a force above a hundredth of the velocity lowered j, and a
+// channel starting from rest took the FP64 form throughout, 1.92 ms a step of
+// 128^3 in place of 0.37).  Error against 128-bit floating point, relative to the
+// node's largest population, rms / max: j lowered by 0 or 1 1.5e-16 / 3.3e-16
 // (FP64 form 2.0e-16 / 5.6e-16), by 2 2.6e-16 / 5.0e-16, by 4 9e-16 / 2.6e-15.
 constexpr int kFxYield = 1;
 __host__ __device__ __forceinline__ bool collide_fx_at(double (&f)[NPOP], bool sum_rho, double& rho,
@@ -865,10 +878,10 @@ __host__ __device__ __forceinline__ bool collide_fx_at(double (&f)[NPOP], bool s
   for (int q = 0; q < NPOP; ++q) ef = most(ef, fx_exponent(f[q]));
   const int eu = most(fx_exponent(ux), most(fx_exponent(uy), fx_exponent(uz)));
   const int eF = most(fx_exponent(fx), most(fx_exponent(fy), fx_exponent(fz)));
-  // |f| < 2^(-4 - j), |u| < 2^(-2 - j), |F| < 2^(-9 - j), |rho| < 2^(-1 - j)
-  // as fixed point: 2^54, 2^62, 2^61, 2^57
+  // |f| < 2^(-4 - j), |u| < 2^(-2 - j), |F| < 2^(-3 - j), |rho| < 2^(-1 - j)
+  // as fixed point: 2^54, 2^62, 2^61, 2^57 (and 0.1 u + 0.05 F in its range)
   const int jf = 1018 - ef;
-  int j = -most(-jf, most(eu - 1020, eF - 1013));
+  int j = -most(-jf, most(eu - 1020, eF - 1019));
   if (!sum_rho) j = -most(-j, fx_exponent(rho) - 1021);
   if (j < 0 || j > 40 || jf - j > kFxYield) return false;
   long long g[NPOP], h[NPOP];
@@ -877,14 +890,15 @@ __host__ __device__ __forceinline__ bool collide_fx_at(double (&f)[NPOP], bool s
   FxSums o;
   fx_sums(g, o);
   const long long u[3] = {fx_from_k(ux, kFxUU + j), fx_from_k(uy, kFxUU + j), fx_from_k(uz, kFxUU + j)};
-  const long long w[3] = {fx_from_k(fx, kFxF + j), fx_from_k(fy, kFxF + j), fx_from_k(fz, kFxF + j)};
+  const long long w[3] = {fx_from_k(fx, kFxWide + j), fx_from_k(fy, kFxWide + j),
+                          fx_from_k(fz, kFxWide + j)};
   const long long half = (1LL << j) >> 1;
   const Split U[3] = {split(u[0]), split(u[1]), split(u[2])};
   const Split V[3] = {split((u[0] + half) >> j), split((u[1] + half) >> j), split((u[2] + half) >> j)};
   const Split Fj[3] = {split(w[0]), split(w[1]), split(w[2])};
   const Split F[3] = {split((w[0] + half) >> j), split((w[1] + half) >> j), split((w[2] + half) >> j)};
   const long long rho_i = sum_rho ? o.rho : fx_from_k(rho, kFxIn + j);
-  if (!fx_relax(o, rho_i, U, V, F, Fj, r, h, 0)) return false;
+  if (!fx_relax<true>(o, rho_i, U, V, F, Fj, r, h, 0)) return false;
   if (sum_rho) rho = fx_to_cvt(o.rho, kFxIn + j);
 #pragma unroll
   for (int q = 0; q < NPOP; ++q) f[q] = fx_to_cvt(h[q], kFxOut + j);

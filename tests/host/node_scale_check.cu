@@ -4,7 +4,8 @@
 // equilibrium and at rest.  Prints per MRT rate set, velocity U and force F
 //   mrt U F states declined ordinary ordinary_declined max_error
 // with the error relative to the node's largest population before or after,
-// and the ordinary states those whose force is below 1/128 of the velocity.
+// and the ordinary states those whose force is below twice their largest
+// population.
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -45,10 +46,9 @@ int main() {
           double g[19], rho9 = rho;
           std::memcpy(g, f, sizeof f);
           ++states;
-          auto largest = [](const double (&a)[3]) {
-            return std::fmax(std::fabs(a[0]), std::fmax(std::fabs(a[1]), std::fabs(a[2])));
-          };
-          const bool plain = 128 * largest(F) < largest(u);
+          double most = 0;
+          for (int q = 0; q < 19; ++q) most = std::fmax(most, std::fabs(f[q]));
+          const bool plain = std::fmax(std::fabs(F[0]), std::fmax(std::fabs(F[1]), std::fabs(F[2]))) < 2 * most;
           ordinary += plain;
           if (!collide_fx_at(g, false, rho9, u[0], u[1], u[2], F[0], F[1], F[2], rt)) {
             ++declined;
