@@ -464,7 +464,7 @@ __global__ void k_stream(Geometry g, const T* __restrict__ fin, T* __restrict__ 
 // declines.  The literal form's ~615 FP64 instructions a node took 1.75 ms at
 // 128^3, two thirds of a step of the subroutine loop there (150 spheres: 2.4
 // -> 0.71 ms a step with this and macrovar's integer sums).  Five CTAs an SM
-// (96 registers, 260 bytes spilled) hide its loads best: that step without
+// (96 registers, 252 bytes spilled) hide its loads best: that step without
 // spheres 458 us, four 474, six 480, three 504.
 template <typename T, bool FX = false>
 __global__ void __launch_bounds__(128, FX ? 5 : 1) k_collision(Geometry g, Rates r, RatesT<double> rt, T* __restrict__ f,
@@ -501,8 +501,8 @@ __global__ void __launch_bounds__(128, FX ? 5 : 1) k_collision(Geometry g, Rates
 // populations as they stand with the largest density change of the iteration
 // that made them, then the next iteration's collision_MRT (velocity held) and
 // streaming into the other buffer: 2 x 19 + 5 values a node instead of the
-// 2 x 42 + 20 of three kernels (128^3: 1.96 -> 0.249 ms; three CTAs an SM 0.253,
-// five 0.291).
+// 2 x 42 + 20 of three kernels (128^3: 1.96 -> 0.253 ms; with three CTAs an
+// SM 1.5 % more, with five 17 %).
 // first: the collision uses the stored density (no iteration made these
 // populations).  before: the change the previous pass found; when it is within
 // eps or not finite the loop has ended, and this pass does nothing.
